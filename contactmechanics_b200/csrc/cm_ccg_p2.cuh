@@ -43,10 +43,9 @@ k_ccg_row_fwd(CcgArgs<R> a) {
   const C* tw = stage_twiddles<LOGN, Sh::LR, Sh::THREADS, Sh::ONEBUF>(tws, a.op.twy);
   pdl_wait();
   CcgState* st = a.st;
-  if (st->done) return;
-  if (MODE == MODE_T && st->branch != 0) return;
   CcgView cv;
   load_view(st, cv);
+  if (cv.done || (MODE == MODE_T && cv.branch != 0)) return;
   __syncthreads();
   const int s = threadIdx.x >> P::LTPS, tt = threadIdx.x & (P::TPS - 1);
   const int tx = a.tx, ty = a.ty, ny = N;
@@ -73,19 +72,29 @@ k_ccg_row_fwd(CcgArgs<R> a) {
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int x0 = tile * ROWS, xa = x0 + 2 * s;
     if (nst > 0) {
-      if (threadIdx.x == 0) {
+      if (threadIdx.x < 32) {
         fence_async_shared();
         fence_async_global();
         const int nr = min(ROWS, tx - x0);
         const unsigned rb = (unsigned)(ty * sizeof(R));
-        mbar_expect_tx(&mbar, (unsigned)(nst * nr) * rb);
+        if (threadIdx.x == 0) mbar_expect_tx(&mbar, (unsigned)(nst * nr) * rb);
+        __syncwarp();
+        // the tile's rows of a topography field are contiguous: one copy per
+        // field (lane j); the displacement's rows only where the domain has no
+        // padding columns, else one copy per row (lane r).  One lane issuing a
+        // copy per row and field took 3000 cycles for 16 rows.
+        const int lane = threadIdx.x;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           if (j >= nst) break;
-          const R* src = j == 0 ? fio : j == jt ? t_io : j == 1 ? u_in : h_in;
-          const int ld = (j == 1 && need_gap) ? ny : ty;
-          for (int r = 0; r < nr; ++r)
-            bulk_g2s(stg + (size_t)(j * ROWS + r) * ty, src + (size_t)(x0 + r) * ld, rb, &mbar);
+          R* dst = stg + (size_t)j * ROWS * ty;
+          if (j == 1 && need_gap && ty != ny) {
+            for (int r = lane; r < nr; r += 32)
+              bulk_g2s(dst + (size_t)r * ty, u_in + (size_t)(x0 + r) * ny, rb, &mbar);
+          } else if (lane == 31 - j) {
+            const R* src = j == 0 ? fio : j == jt ? t_io : j == 1 ? u_in : h_in;
+            bulk_g2s(dst, src + (size_t)x0 * ty, (unsigned)nr * rb, &mbar);
+          }
         }
       }
       const bool ok = __syncthreads_and(mbar_wait(&mbar, mphase)) != 0;
@@ -192,13 +201,13 @@ k_ccg_row_fwd(CcgArgs<R> a) {
   if (MODE == MODE_T) {
     double vr[1] = {acc};
     const int kinds[1] = {RED_SUM};
-    tile_finish<1>(a.partials, a.counter, blockIdx.x, gridDim.x, vr, kinds,
-                   [&](double (&r)[1]) { st->sum_cgt = r[0]; });
+    tile_finish<1>(st, a.partials, a.counter, blockIdx.x, gridDim.x, vr, kinds,
+                   [&](CcgState& s, double (&r)[1]) { s.sum_cgt = r[0]; });
   } else {
     double vr[2] = {acc, (double)amax};
     const int kinds[2] = {RED_SUM, RED_MAX};
-    tile_finish<2>(a.partials, a.counter, blockIdx.x, gridDim.x, vr, kinds,
-                   [&](double (&r)[2]) { fin_force(*st, r); });
+    tile_finish<2>(st, a.partials, a.counter, blockIdx.x, gridDim.x, vr, kinds,
+                   [&](CcgState& s, double (&r)[2]) { fin_force(s, r); });
   }
 }
 
@@ -224,10 +233,9 @@ k_ccg_row_inv(CcgArgs<R> a) {
   const C* tw = stage_twiddles<LOGN, Sh::LR, Sh::THREADS, Sh::ONEBUF>(tws, a.op.twy);
   pdl_wait();
   CcgState* st = a.st;
-  if (st->done) return;
-  if (MODE == MODE_T && st->branch != 0) return;
   CcgView cv;
   load_view(st, cv);
+  if (cv.done || (MODE == MODE_T && cv.branch != 0)) return;
   __syncthreads();
   const int s = threadIdx.x >> P::LTPS, tt = threadIdx.x & (P::TPS - 1);
   const int tx = a.tx, ty = a.ty, nx = a.op.nx;
@@ -274,11 +282,19 @@ k_ccg_row_inv(CcgArgs<R> a) {
     fft_len<C, true, LOGN, Sh::LR, Sh::ONEBUF, Sh::ONESTG>(v, bufA, bufB, s * N, 1, tt, tw);
     if (MODE == MODE_T) {
 #pragma unroll
-      for (int q = 0; q < Sh::E; ++q) {
-        const int y = tt + q * P::TPS;
-        if (y >= ty) continue;
-        if (xa < tx) a0 += (double)v[q].x * (double)t_in[(size_t)xa * ty + y];
-        if (xa + 1 < tx) a0 += (double)v[q].y * (double)t_in[(size_t)(xa + 1) * ty + y];
+      for (int w = 0; w < 2; ++w) {
+        const int x = xa + w;
+        if (x >= tx) continue;
+        const R* __restrict__ trow = t_in + (size_t)x * ty;
+        R tv[Sh::E];
+#pragma unroll
+        for (int q = 0; q < Sh::E; ++q) {
+          const int y = tt + q * P::TPS;
+          tv[q] = trow[y < ty ? y : 0];
+        }
+#pragma unroll
+        for (int q = 0; q < Sh::E; ++q)
+          if (tt + q * P::TPS < ty) a0 += (double)(w ? v[q].y : v[q].x) * (double)tv[q];
       }
     } else {
       // u on the whole domain, max |du| and the maximum penetration; on the
@@ -290,23 +306,35 @@ k_ccg_row_inv(CcgArgs<R> a) {
       for (int w = 0; w < 2; ++w) {
         const int x = xa + w;
         if (x >= rows_total) continue;
-        // every input of the row's E elements first, then the stores
-        R uo[Sh::E], hv[Sh::E], fn[Sh::E];
-        bool cc[Sh::E];
+        // every input of the row's E elements first, from addresses that are
+        // valid without a test (a branch around each load, or a use of one
+        // inside it, makes the row's loads wait for one another: 8700 cycles a
+        // tile of 16 x 256 in FP64 instead of 2500), then the stores
+        const bool in_x = x < tx;
+        R uo[Sh::E], hv[Sh::E], fn[Sh::E], fa[Sh::E];
 #pragma unroll
-        for (int q = 0; q < Sh::E; ++q) {
-          const int y = tt + q * P::TPS;
-          hv[q] = 0; fn[q] = 0; cc[q] = false;
-          uo[q] = u_io[(size_t)x * N + y];
-          if (x < tx && y < ty) {
-            const size_t ic = (size_t)x * ty + y;
+        for (int q = 0; q < Sh::E; ++q) uo[q] = u_io[(size_t)x * N + tt + q * P::TPS];
+        if (in_x) {
+          const size_t rb = (size_t)x * ty;
+#pragma unroll
+          for (int q = 0; q < Sh::E; ++q) {
+            const int y = tt + q * P::TPS;
+            const size_t ic = rb + (y < ty ? y : 0);
             hv[q] = h_in[ic];
             fn[q] = fn_buf[ic];
-            if (cv.branch == 0) {
-              const R fa = fa_buf[ic];
-              cc[q] = (fa < 0) && (!cv.has_h || fa > hdn);
-            } else {
-              cc[q] = gneg[ic] != 0;
+          }
+          // the force at the iteration's start, or the mixing step's mask
+          if (cv.branch == 0) {
+#pragma unroll
+            for (int q = 0; q < Sh::E; ++q) {
+              const int y = tt + q * P::TPS;
+              fa[q] = fa_buf[rb + (y < ty ? y : 0)];
+            }
+          } else {
+#pragma unroll
+            for (int q = 0; q < Sh::E; ++q) {
+              const int y = tt + q * P::TPS;
+              fa[q] = (R)gneg[rb + (y < ty ? y : 0)];
             }
           }
         }
@@ -316,9 +344,10 @@ k_ccg_row_inv(CcgArgs<R> a) {
           const R val = w ? v[q].y : v[q].x;
           du = fmax(du, fabs(val - uo[q]));
           u_io[(size_t)x * N + y] = val;
-          if (x < tx && y < ty) {
+          if (in_x && y < ty) {
+            const bool cc = cv.branch == 0 ? (fa[q] < 0) && (!cv.has_h || fa[q] > hdn) : fa[q] != 0;
             const R pen = (hv[q] + off) - val;
-            pmax = fmax(pmax, cc[q] ? pen : (R)0);
+            pmax = fmax(pmax, cc ? pen : (R)0);
             const bool c0 = fn[q] < 0;
             const bool c = c0 && (!cv.has_h || fn[q] > hdn);
             const R g = val - hv[q];
@@ -340,28 +369,29 @@ k_ccg_row_inv(CcgArgs<R> a) {
   if (MODE == MODE_T) {
     double vr[1] = {a0};
     const int kinds[1] = {RED_SUM};
-    tile_finish<1>(a.partials, a.counter, blockIdx.x, gridDim.x, vr, kinds,
-                   [&](double (&r)[1]) { fin_tau(*st, r); });
+    tile_finish<1>(st, a.partials, a.counter, blockIdx.x, gridDim.x, vr, kinds,
+                   [&](CcgState& s, double (&r)[1]) { fin_tau(s, r); });
   } else {
     double vr[8] = {(double)du, (double)pmax, (double)n_c, (double)n_cg, s_cg, (double)gmax,
                     (double)gmin, s_cg2};
     const int kinds[8] = {RED_MAX, RED_MAX, RED_SUM, RED_SUM, RED_SUM, RED_MAX, RED_MIN, RED_SUM};
     const int fuse = a.fuse_gsum;
-    tile_finish<8>(a.partials, a.counter, blockIdx.x, gridDim.x, vr, kinds, [&](double (&r)[8]) {
-      ccg_converge(*st, r[0], r[1]);
-      if (!st->done) {
+    tile_finish<8>(st, a.partials, a.counter, blockIdx.x, gridDim.x, vr, kinds,
+                   [&](CcgState& s, double (&r)[8]) {
+      ccg_converge(s, r[0], r[1]);
+      if (!s.done) {
         double b[5] = {r[2], r[3], r[4], r[5], r[6]};
-        fin_begin(*st, b);
-        if (fuse && st->branch == 0) {
+        fin_begin(s, b);
+        if (fuse && s.branch == 0) {
           // G = sum over c of (g - offset)^2 from the sums over c of g^2
           // and g (each g^2 of an FP32 gap is exact in FP64); near
           // convergence this loses about eps64 * sum g^2 / G, far below the
           // FP32 gaps' own rounding
-          const double off = st->offset;
-          double G = r[7] - 2.0 * off * r[4] + (double)st->A_cg * off * off;
+          const double off = s.offset;
+          double G = r[7] - 2.0 * off * r[4] + (double)s.A_cg * off * off;
           if (G < 0) G = 0;  // rounding (a NaN stays NaN)
           double gv[1] = {G};
-          fin_gsum(*st, gv);
+          fin_gsum(s, gv);
         }
       }
     });
@@ -434,11 +464,13 @@ __global__ void __launch_bounds__(CM_EW_THREADS) k_ew_gsum(CcgArgs<R> a) {
   pdl_trigger();
   pdl_wait();
   CcgState* st = a.st;
-  if (st->done || st->branch != 0) return;
-  const int has_h = st->p.has_h;
-  const R hdn = neg_down<R>(st->p.H);
-  const R off = (R)st->offset;
-  const R* __restrict__ f = a.f[st->parity & 1];
+  CcgView cv;
+  load_view(st, cv);
+  if (cv.done || cv.branch != 0) return;
+  const int has_h = cv.has_h;
+  const R hdn = neg_down<R>(cv.H);
+  const R off = (R)cv.offset;
+  const R* __restrict__ f = a.f[cv.par & 1];
   const R* __restrict__ u = a.u;
   const R* __restrict__ h = a.h;
   double G = 0;
@@ -472,8 +504,8 @@ __global__ void __launch_bounds__(CM_EW_THREADS) k_ew_gsum(CcgArgs<R> a) {
   }
   double v[1] = {G};
   const int kinds[1] = {RED_SUM};
-  tile_finish<1>(a.partials, a.counter, blockIdx.x, gridDim.x, v, kinds,
-                 [&](double (&r)[1]) { fin_gsum(*st, r); });
+  tile_finish<1>(st, a.partials, a.counter, blockIdx.x, gridDim.x, v, kinds,
+                 [&](CcgState& s, double (&r)[1]) { fin_gsum(s, r); });
 }
 
 // Force update, projection onto [0, H] and the constraint bookkeeping
@@ -487,12 +519,14 @@ __global__ void __launch_bounds__(CM_EW_THREADS) k_ew_update(CcgArgs<R> a) {
   pdl_trigger();
   pdl_wait();
   CcgState* st = a.st;
-  if (st->done) return;
-  const int par = st->parity & 1, has_h = st->p.has_h, branch = st->branch;
-  const double H = st->p.H;
-  const R off = (R)st->offset;
-  const R tau = (R)st->tau;
+  CcgView cv;
+  load_view(st, cv);
   const double mix = st->cur_mixfac;
+  if (cv.done) return;
+  const int par = cv.par & 1, has_h = cv.has_h, branch = cv.branch;
+  const double H = cv.H;
+  const R off = (R)cv.offset;
+  const R tau = (R)cv.tau;
   const R* __restrict__ f = a.f[par];
   R* __restrict__ fo = a.f[par ^ 1];
   const R* __restrict__ t = a.t;
@@ -560,6 +594,6 @@ __global__ void __launch_bounds__(CM_EW_THREADS) k_ew_update(CcgArgs<R> a) {
   }
   double v[5] = {(double)a_fl, (double)min_fn + H, (double)max_t, s_fp, (double)n_nc};
   const int kinds[5] = {RED_SUM, RED_MIN, RED_MAX, RED_SUM, RED_SUM};
-  tile_finish<5>(a.partials, a.counter, blockIdx.x, gridDim.x, v, kinds,
-                 [&](double (&r)[5]) { fin_update(*st, r); });
+  tile_finish<5>(st, a.partials, a.counter, blockIdx.x, gridDim.x, v, kinds,
+                 [&](CcgState& s, double (&r)[5]) { fin_update(s, r); });
 }

@@ -63,6 +63,15 @@ template <typename C, typename R> CM_DEVINL C cmake(R x, R y) { C r; r.x = x; r.
 CM_DEVINL void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 CM_DEVINL void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// The ticket of a block that has written its results: the block's thread that
+// takes it releases its own earlier writes, and sees those of every block
+// whose ticket came before.
+CM_DEVINL unsigned take_ticket(unsigned* counter) {
+  unsigned prev;
+  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(prev) : "l"(counter) : "memory");
+  return prev;
+}
+
 #define CM_BARRIER_TIMEOUT_CYCLES 4000000000LL  // about two seconds
 
 // ---------------------------------------------------------------------------
@@ -170,36 +179,78 @@ CM_DEVINL double red_apply(int kind, double a, double b) {
   return kind == RED_SUM ? a + b : (kind == RED_MAX ? fmax(a, b) : fmin(a, b));
 }
 
-// Reduce NV doubles across the block with a fixed tree (deterministic).
-// kinds[i] selects sum / max / min.  Result valid in thread 0.
-// `sm` must hold 32*NV doubles.  All threads must call.
-template <int NV>
-CM_DEVINL void block_reduce(double (&v)[NV], const int (&kinds)[NV], double* sm) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nw = (blockDim.x + 31) >> 5;
+// Butterfly over the lanes of a warp on N values per lane, steps O, O/2 .. 1.
+// While a lane holds more than one value it keeps half of them and hands the
+// other half to its partner, so 8 values take 4 + 2 + 1 + 1 + 1 shuffles
+// instead of 8 x 5.  Every value still meets its 32 lanes in the order of the
+// plain xor tree 16, 8, 4, 2, 1.  mx: maximum (else sum).
+template <int N, int O>
+CM_DEVINL void warp_fold(double* w, bool* mx) {
+  if constexpr (O > 0) {
+    if constexpr (N > 1) {
+      constexpr int H = N / 2;
+      const bool up = (threadIdx.x & O) != 0;  // this lane keeps the upper half
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-      v[i] = red_apply(kinds[i], v[i], __shfl_xor_sync(0xffffffffu, v[i], o));
-  }
-  __syncthreads();
-  if (lane == 0) {
-#pragma unroll
-    for (int i = 0; i < NV; ++i) sm[i * 32 + warp] = v[i];
-  }
-  __syncthreads();
-  if (warp == 0) {
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      double x = lane < nw ? sm[i * 32 + lane] : red_neutral(kinds[i]);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1)
-        x = red_apply(kinds[i], x, __shfl_xor_sync(0xffffffffu, x, o));
-      v[i] = x;
+      for (int i = 0; i < H; ++i) {
+        const double keep = up ? w[H + i] : w[i], give = up ? w[i] : w[H + i];
+        const double got = __shfl_xor_sync(0xffffffffu, give, O);
+        mx[i] = up ? mx[H + i] : mx[i];
+        w[i] = mx[i] ? fmax(keep, got) : keep + got;
+      }
+      warp_fold<H, O / 2>(w, mx);
+    } else {
+      const double got = __shfl_xor_sync(0xffffffffu, w[0], O);
+      w[0] = mx[0] ? fmax(w[0], got) : w[0] + got;
+      warp_fold<1, O / 2>(w, mx);
     }
   }
+}
+
+// Reduce NV doubles across the block with a fixed tree (deterministic).
+// kinds[i] selects sum / max / min (a minimum is the maximum of the negated
+// values).  The result is valid in every thread.  `sm` must hold 32*NV
+// doubles.  All threads must call; whole warps only.  It ends every reducing
+// pass, alone on the critical path: with one value after the other (40
+// dependent shuffles of a double for 8 values, twice, the second time on one
+// warp) the 8 values of the displacement pass took 2600 cycles.
+template <int NV>
+CM_DEVINL void block_reduce(double (&v)[NV], const int (&kinds)[NV], double* sm) {
+  constexpr int LNP = NV <= 1 ? 0 : NV <= 2 ? 1 : NV <= 4 ? 2 : NV <= 8 ? 3 : NV <= 16 ? 4 : 5;
+  constexpr int NP = 1 << LNP, SPAN = 32 / NP;  // lanes that end up with one value
+  static_assert(NV <= 32, "one value per lane at most");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nw = blockDim.x >> 5;
+  double w[NP];
+  bool mx[NP];
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    w[i] = i < NV ? (kinds[i < NV ? i : 0] == RED_MIN ? -v[i < NV ? i : 0] : v[i < NV ? i : 0]) : 0.0;
+    mx[i] = i < NV && kinds[i < NV ? i : 0] != RED_SUM;
+  }
+  warp_fold<NP, 16>(w, mx);
   __syncthreads();
+  const int mine = lane / SPAN;  // the value this lane holds
+  if (lane % SPAN == 0 && mine < NV) sm[mine * 32 + warp] = w[0];
+  __syncthreads();
+  if (nw > 1) {
+    // value i over the warps: by warp i, in the order of the same tree
+    for (int i = warp; i < NV; i += nw) {
+      bool is_max = false;
+#pragma unroll
+      for (int k = 0; k < NV; ++k)
+        if (k == i) is_max = kinds[k] != RED_SUM;
+      double x = lane < nw ? sm[i * 32 + lane] : (is_max ? -INFINITY : 0.0);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const double got = __shfl_xor_sync(0xffffffffu, x, o);
+        x = is_max ? fmax(x, got) : x + got;
+      }
+      if (lane == 0) sm[i * 32] = x;
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < NV; ++i) v[i] = kinds[i] == RED_MIN ? -sm[i * 32] : sm[i * 32];
 }
 
 // Loop over e in [0, n) with the block's threads, U indices per thread per

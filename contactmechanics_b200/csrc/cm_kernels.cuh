@@ -42,23 +42,35 @@ CM_DEVINL size_t spec_at(int x, int k, int nx, int lw) {
 // ---------------------------------------------------------------------------
 // last-tile reduction
 // ---------------------------------------------------------------------------
+// Every block leaves one partial of NV values; the last one to finish (atomic
+// ticket) reduces them in a fixed order and runs the scalar step `fin(s, a)`
+// on the solve's state.  The tail is a chain of latencies on one block while
+// the rest of the chip waits, so the state travels as a whole: the block's
+// threads bring it into shared memory together with the partials (one L2
+// round trip), thread 0 works on that copy, and the threads write it back.  Read
+// and written field by field in global memory, the convergence step alone
+// was a dozen dependent L2 accesses.
+// tile_finish_warp hands the copy to the whole of warp 0; tile_finish to its
+// first lane.
 template <int NV, typename Fin>
-CM_DEVINL void tile_finish(double* __restrict__ partials, unsigned int* counter, int tile,
-                           int ntiles, double (&v)[NV], const int (&kinds)[NV], Fin fin) {
+CM_DEVINL void tile_finish_warp(CcgState* __restrict__ st, double* __restrict__ partials,
+                                unsigned int* counter, int tile, int ntiles, double (&v)[NV],
+                                const int (&kinds)[NV], Fin fin) {
   __shared__ double red_sm[32 * NV];
+  __shared__ __align__(16) unsigned char st_sm[sizeof(CcgState)];
   __shared__ int am_last;
   block_reduce<NV>(v, kinds, red_sm);
   if (threadIdx.x == 0) {
     double* P = partials + (size_t)tile * NV;
 #pragma unroll
     for (int i = 0; i < NV; ++i) P[i] = v[i];
-    __threadfence();
-    const unsigned prev = atomicAdd(counter, 1u);
-    am_last = (prev == (unsigned)(ntiles - 1));
+    am_last = (take_ticket(counter) == (unsigned)(ntiles - 1));
   }
   __syncthreads();
   if (!am_last) return;
-  __threadfence();
+  constexpr int NW = (int)(sizeof(CcgState) / sizeof(int4));
+  for (int i = threadIdx.x; i < NW; i += blockDim.x)
+    reinterpret_cast<int4*>(st_sm)[i] = __ldcg(reinterpret_cast<const int4*>(st) + i);
   double acc[NV];
 #pragma unroll
   for (int i = 0; i < NV; ++i) acc[i] = red_neutral(kinds[i]);
@@ -67,11 +79,22 @@ CM_DEVINL void tile_finish(double* __restrict__ partials, unsigned int* counter,
     for (int i = 0; i < NV; ++i)
       acc[i] = red_apply(kinds[i], acc[i], __ldcg(partials + (size_t)tt * NV + i));
   }
-  block_reduce<NV>(acc, kinds, red_sm);
-  if (threadIdx.x == 0) {
-    fin(acc);
-    *counter = 0;
-  }
+  block_reduce<NV>(acc, kinds, red_sm);  // its barriers also publish the state's copy
+  if (threadIdx.x < 32) fin(*reinterpret_cast<CcgState*>(st_sm), acc);
+  if (threadIdx.x == 0) *counter = 0;
+  __syncthreads();
+  for (int i = threadIdx.x; i < NW; i += blockDim.x)
+    reinterpret_cast<int4*>(st)[i] = reinterpret_cast<const int4*>(st_sm)[i];
+}
+
+template <int NV, typename Fin>
+CM_DEVINL void tile_finish(CcgState* __restrict__ st, double* __restrict__ partials,
+                           unsigned int* counter, int tile, int ntiles, double (&v)[NV],
+                           const int (&kinds)[NV], Fin fin) {
+  tile_finish_warp<NV>(st, partials, counter, tile, ntiles, v, kinds,
+                       [&](CcgState& s, double (&a)[NV]) {
+                         if (threadIdx.x == 0) fin(s, a);
+                       });
 }
 
 #ifndef CM_BARRIER_SLEEP_NS
@@ -144,11 +167,13 @@ template <> CM_DEVINL double neg_down<double>(double H) { return -H; }
 
 // scalar state of a contact solve that the operator prologues/epilogues use
 struct CcgView {
-  int par, has_h, uniform, apply_nc, branch;
+  int done, par, has_h, uniform, apply_nc, branch;
   double beta, offset, H, scale, tau, funif;
 };
 
+// (every field in one batch of loads, before any test of them)
 CM_DEVINL void load_view(const CcgState* st, CcgView& v) {
+  v.done = st->done;
   v.par = st->parity;
   v.has_h = st->p.has_h;
   v.uniform = st->uniform;
@@ -450,9 +475,8 @@ k_row_fwd(const Slot<R>* __restrict__ slots, const int2* __restrict__ items) {
   CcgState* st = Sp->st;
   CcgView cv{};
   if (MODE == MODE_T || MODE == MODE_F) {
-    if (st->done) return;
-    if (MODE == MODE_T && st->branch != 0) return;
     load_view(st, cv);
+    if (cv.done || (MODE == MODE_T && cv.branch != 0)) return;
   }
   const int ny = Sp->ny;
   C* tws = reinterpret_cast<C*>(smem_raw);
@@ -464,13 +488,13 @@ k_row_fwd(const Slot<R>* __restrict__ slots, const int2* __restrict__ items) {
   if (MODE == MODE_T) {
     double v[1] = {acc};
     const int kinds[1] = {RED_SUM};
-    tile_finish<1>(Sp->partials, Sp->counter, item.y, Sp->nt_rowt, v, kinds,
-                   [&](double (&a)[1]) { st->sum_cgt = a[0]; });
+    tile_finish<1>(st, Sp->partials, Sp->counter, item.y, Sp->nt_rowt, v, kinds,
+                   [&](CcgState& s, double (&a)[1]) { s.sum_cgt = a[0]; });
   } else if (MODE == MODE_F) {
     double v[2] = {acc, amax};
     const int kinds[2] = {RED_SUM, RED_MAX};
-    tile_finish<2>(Sp->partials, Sp->counter, item.y, Sp->nt_rowt, v, kinds,
-                   [&](double (&a)[2]) { fin_force(*st, a); });
+    tile_finish<2>(st, Sp->partials, Sp->counter, item.y, Sp->nt_rowt, v, kinds,
+                   [&](CcgState& s, double (&a)[2]) { fin_force(s, a); });
   }
 }
 
@@ -716,9 +740,8 @@ k_row_inv(const Slot<R>* __restrict__ slots, const int2* __restrict__ items) {
   CcgState* st = Sp->st;
   CcgView cv{};
   if (MODE == MODE_T || MODE == MODE_F) {
-    if (st->done) return;
-    if (MODE == MODE_T && st->branch != 0) return;
     load_view(st, cv);
+    if (cv.done || (MODE == MODE_T && cv.branch != 0)) return;
   }
   const int ny = Sp->ny;
   C* tws = reinterpret_cast<C*>(smem_raw);
@@ -730,13 +753,13 @@ k_row_inv(const Slot<R>* __restrict__ slots, const int2* __restrict__ items) {
   if (MODE == MODE_T) {
     double v[1] = {a0};
     const int kinds[1] = {RED_SUM};
-    tile_finish<1>(Sp->partials, Sp->counter, item.y, Sp->nt_rowt, v, kinds,
-                   [&](double (&a)[1]) { fin_tau(*st, a); });
+    tile_finish<1>(st, Sp->partials, Sp->counter, item.y, Sp->nt_rowt, v, kinds,
+                   [&](CcgState& s, double (&a)[1]) { fin_tau(s, a); });
   } else if (MODE == MODE_F) {
     double v[2] = {a0, a1};
     const int kinds[2] = {RED_MAX, RED_MAX};
-    tile_finish<2>(Sp->partials, Sp->counter, item.y, Sp->nt_rowd, v, kinds,
-                   [&](double (&a)[2]) { ccg_converge(*st, a[0], a[1]); });
+    tile_finish<2>(st, Sp->partials, Sp->counter, item.y, Sp->nt_rowd, v, kinds,
+                   [&](CcgState& s, double (&a)[2]) { ccg_converge(s, a[0], a[1]); });
   }
 }
 
@@ -835,8 +858,8 @@ k_ccg_begin(const Slot<R>* __restrict__ slots, const int2* __restrict__ items, i
     begin_tile<R>(Sp, tile, f, has_h, hdn, a_c, a_cg, s_cg, gmax, gmin);
   double v[5] = {(double)a_c, (double)a_cg, s_cg, (double)gmax, (double)gmin};
   const int kinds[5] = {RED_SUM, RED_SUM, RED_SUM, RED_MAX, RED_MIN};
-  tile_finish<5>(Sp->partials, Sp->counter, W.part, W.nparts, v, kinds,
-                 [&](double (&a)[5]) { fin_begin(*st, a); });
+  tile_finish<5>(st, Sp->partials, Sp->counter, W.part, W.nparts, v, kinds,
+                 [&](CcgState& s, double (&a)[5]) { fin_begin(s, a); });
 }
 
 // G over one comp tile: sum over the CG area of g^2.
@@ -880,8 +903,8 @@ k_ccg_gsum(const Slot<R>* __restrict__ slots, const int2* __restrict__ items, in
   for (int tile = W.first; tile < W.end; tile += W.step) gsum_tile<R>(Sp, tile, f, has_h, hdn, off, G);
   double v[1] = {G};
   const int kinds[1] = {RED_SUM};
-  tile_finish<1>(Sp->partials, Sp->counter, W.part, W.nparts, v, kinds,
-                 [&](double (&a)[1]) { fin_gsum(*st, a); });
+  tile_finish<1>(st, Sp->partials, Sp->counter, W.part, W.nparts, v, kinds,
+                 [&](CcgState& s, double (&a)[1]) { fin_gsum(s, a); });
 }
 
 // One pass of the load-controlled offset bisection of the mixing step
@@ -946,8 +969,8 @@ k_ccg_bisect(const Slot<R>* __restrict__ slots, const int2* __restrict__ items, 
   int kinds[CM_BIS_CAND];
 #pragma unroll
   for (int i = 0; i < CM_BIS_CAND; ++i) kinds[i] = RED_SUM;
-  tile_finish<CM_BIS_CAND>(Sp->partials, Sp->counter, W.part, W.nparts, cnt, kinds,
-                           [&](double (&a)[CM_BIS_CAND]) { fin_bisect(*st, a); });
+  tile_finish<CM_BIS_CAND>(st, Sp->partials, Sp->counter, W.part, W.nparts, cnt, kinds,
+                           [&](CcgState& s, double (&a)[CM_BIS_CAND]) { fin_bisect(s, a); });
 }
 
 // All the bisection passes of one iteration in one launch (single solves):
@@ -1019,8 +1042,8 @@ k_ccg_bisect_passes(const Slot<R>* __restrict__ slots, const int2* __restrict__ 
     int kinds[CM_BIS_CAND];
 #pragma unroll
     for (int i = 0; i < CM_BIS_CAND; ++i) kinds[i] = RED_SUM;
-    tile_finish<CM_BIS_CAND>(Sp->partials, Sp->counter, blockIdx.x, gridDim.x, cnt, kinds,
-                             [&](double (&a)[CM_BIS_CAND]) { fin_bisect(*st, a); });
+    tile_finish<CM_BIS_CAND>(st, Sp->partials, Sp->counter, blockIdx.x, gridDim.x, cnt, kinds,
+                             [&](CcgState& s, double (&a)[CM_BIS_CAND]) { fin_bisect(s, a); });
     if (!grid_barrier(bar, gen, &ok_sm)) {
       if (threadIdx.x == 0) {
         st->status = CMS_TIMEOUT;
@@ -1106,8 +1129,8 @@ k_ccg_update(const Slot<R>* __restrict__ slots, const int2* __restrict__ items, 
     update_tile<R>(Sp, tile, f, fo, has_h, branch, H, hdn, off, tau, mix, A);
   double v[5] = {(double)A.a_fl, (double)A.min_fn + H, (double)A.max_t, A.s_fp, (double)A.n_nc};
   const int kinds[5] = {RED_SUM, RED_MIN, RED_MAX, RED_SUM, RED_SUM};
-  tile_finish<5>(Sp->partials, Sp->counter, W.part, W.nparts, v, kinds,
-                 [&](double (&a)[5]) { fin_update(*st, a); });
+  tile_finish<5>(st, Sp->partials, Sp->counter, W.part, W.nparts, v, kinds,
+                 [&](CcgState& s, double (&a)[5]) { fin_update(s, a); });
 }
 
 // ---------------------------------------------------------------------------

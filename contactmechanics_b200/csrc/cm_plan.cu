@@ -358,8 +358,8 @@ k_h_prep(const Slot<R>* __restrict__ slots, const int2* __restrict__ items, cons
   h_prep_tile<R>(Sp, item.y, h64 ? h64 : Sp->h64, v[0], v[1], v[2]);
   const int kinds[3] = {RED_MAX, RED_MIN, RED_SUM};
   CcgState* st = Sp->st;
-  tile_finish<3>(Sp->partials, Sp->counter, item.y, Sp->nt_comp, v, kinds,
-                 [&](double (&a)[3]) { fin_h_prep(*st, a); });
+  tile_finish<3>(st, Sp->partials, Sp->counter, item.y, Sp->nt_comp, v, kinds,
+                 [&](CcgState& s, double (&a)[3]) { fin_h_prep(s, a); });
 }
 
 // rms height and the default penetration tolerance; pentol_auto < 0: from
@@ -375,9 +375,10 @@ k_h_var(const Slot<R>* __restrict__ slots, const int2* __restrict__ items, const
   h_var_tile<R>(Sp, item.y, h64 ? h64 : Sp->h64, st->sum_cg / st->p.n_surface, v[0]);
   const int kinds[1] = {RED_SUM};
   const int tx = Sp->tx, ty = Sp->ty;
-  tile_finish<1>(Sp->partials, Sp->counter, item.y, Sp->nt_comp, v, kinds, [&](double (&a)[1]) {
-    const int automatic = pentol_auto >= 0 ? pentol_auto : (st->p.pentol <= 0);
-    fin_h_var(*st, a, automatic, rel_pentol, tx, ty);
+  tile_finish<1>(st, Sp->partials, Sp->counter, item.y, Sp->nt_comp, v, kinds,
+                 [&](CcgState& s, double (&a)[1]) {
+    const int automatic = pentol_auto >= 0 ? pentol_auto : (s.p.pentol <= 0);
+    fin_h_var(s, a, automatic, rel_pentol, tx, ty);
   });
 }
 
@@ -431,8 +432,8 @@ k_ccg_result_slots(const Slot<R>* __restrict__ slots, const int2* __restrict__ i
   result_tile<R>(Sp, item.y, st->parity, st->p.has_h, st->branch == 1, st->p.H, Sp->jac_out,
                  Sp->act_out, Sp->pl_out, v);
   const int kinds[4] = {RED_SUM, RED_SUM, RED_SUM, RED_SUM};
-  tile_finish<4>(Sp->partials, Sp->counter, item.y, Sp->nt_comp, v, kinds,
-                 [&](double (&a)[4]) { fin_result(*st, a); });
+  tile_finish<4>(st, Sp->partials, Sp->counter, item.y, Sp->nt_comp, v, kinds,
+                 [&](CcgState& s, double (&a)[4]) { fin_result(s, a); });
 }
 
 // Lockstep batches: the displacement of a row tile's domain rows to FP64
@@ -476,8 +477,8 @@ k_ccg_result(const Slot<R>* __restrict__ slots, const int2* __restrict__ items, 
   result_tile<R>(Sp, item.y, st->parity, st->p.has_h, st->branch == 1, st->p.H, jac, active,
                  plastic, v);
   const int kinds[4] = {RED_SUM, RED_SUM, RED_SUM, RED_SUM};
-  tile_finish<4>(Sp->partials, Sp->counter, item.y, Sp->nt_comp, v, kinds,
-                 [&](double (&a)[4]) { fin_result(*st, a); });
+  tile_finish<4>(st, Sp->partials, Sp->counter, item.y, Sp->nt_comp, v, kinds,
+                 [&](CcgState& s, double (&a)[4]) { fin_result(s, a); });
 }
 
 template <typename R>

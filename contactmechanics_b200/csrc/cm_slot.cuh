@@ -37,7 +37,8 @@ struct CcgParams {
   int maxiter;
 };
 
-struct CcgState {
+// (read and written by the kernels in 16-byte words)
+struct alignas(16) CcgState {
   CcgParams p;
   int it;        // iteration being computed (1-based)
   int done;
