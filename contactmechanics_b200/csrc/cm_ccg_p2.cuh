@@ -281,20 +281,24 @@ k_ccg_row_inv(CcgArgs<R> a) {
     }
     fft_len<C, true, LOGN, Sh::LR, Sh::ONEBUF, Sh::ONESTG>(v, bufA, bufB, s * N, 1, tt, tw);
     if (MODE == MODE_T) {
+      // t of up to 8 elements of both rows in one batch of loads
+      constexpr int CH = Sh::E % 8 == 0 ? 8 : 4;
+      const size_t ra = xa < tx ? (size_t)xa * ty : 0, rb = xa + 1 < tx ? ra + ty : 0;
 #pragma unroll
-      for (int w = 0; w < 2; ++w) {
-        const int x = xa + w;
-        if (x >= tx) continue;
-        const R* __restrict__ trow = t_in + (size_t)x * ty;
-        R tv[Sh::E];
+      for (int q0 = 0; q0 < Sh::E; q0 += CH) {
+        R ta[CH], tb[CH];
 #pragma unroll
-        for (int q = 0; q < Sh::E; ++q) {
-          const int y = tt + q * P::TPS;
-          tv[q] = trow[y < ty ? y : 0];
+        for (int q = 0; q < CH; ++q) {
+          const int y = tt + (q0 + q) * P::TPS, yy = y < ty ? y : 0;
+          ta[q] = t_in[ra + yy];
+          tb[q] = t_in[rb + yy];
         }
 #pragma unroll
-        for (int q = 0; q < Sh::E; ++q)
-          if (tt + q * P::TPS < ty) a0 += (double)(w ? v[q].y : v[q].x) * (double)tv[q];
+        for (int q = 0; q < CH; ++q) {
+          if (tt + (q0 + q) * P::TPS >= ty) continue;
+          if (xa < tx) a0 += (double)v[q0 + q].x * (double)ta[q];
+          if (xa + 1 < tx) a0 += (double)v[q0 + q].y * (double)tb[q];
+        }
       }
     } else {
       // u on the whole domain, max |du| and the maximum penetration; on the

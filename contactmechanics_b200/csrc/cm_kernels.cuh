@@ -577,7 +577,13 @@ k_col(const Slot<R>* __restrict__ slots, const int2* __restrict__ items) {
 
 // Convergence test at the end of an iteration (ConstrainedConjugateGradients.py
 // :391-434, 491-492); run by the last tile of the displacement update.
-CM_DEVINL void ccg_converge(CcgState& s, double maxdu_in, double maxpen_in) {
+// cq: the quotients it needs, (tf - F) / tf (or against the last total force),
+// the relative change of the maximum height, and G / A_cg.
+struct ConvergeQuotients {
+  double rel_tf, rel_mh, g_mean;
+};
+CM_DEVINL void ccg_converge_q(CcgState& s, double maxdu_in, double maxpen_in,
+                              const ConvergeQuotients& cq) {
   // convergence test (ConstrainedConjugateGradients.py:391-434, 491-492)
   const CcgParams& P = s.p;
   s.rep_area = s.A_contact;
@@ -587,16 +593,16 @@ CM_DEVINL void ccg_converge(CcgState& s, double maxdu_in, double maxpen_in) {
   s.maxdu = maxdu_in;
   s.nfev += (s.branch == 0) ? 2 : 1;
   s.G_old = s.G;
-  s.rms_pen = (s.A_cg > 0) ? sqrt(s.G / (double)s.A_cg) : sqrt(s.G);
+  s.rms_pen = sqrt((s.A_cg > 0) ? cq.g_mean : s.G);
   s.max_pen = fmax(0.0, maxpen_in);
   const double tf = s.total_force;
   bool conv = true;
-  if (P.load_control) conv = conv && fabs((tf - P.F) / tf) < P.thermotol;
-  else if (s.have_last_tf) conv = conv && fabs((tf - s.last_tf) / tf) < P.thermotol;
+  if (P.load_control) conv = conv && fabs(cq.rel_tf) < P.thermotol;
+  else if (s.have_last_tf) conv = conv && fabs(cq.rel_tf) < P.thermotol;
   s.last_tf = tf;
   s.have_last_tf = 1;
   const double mh = P.max_surface + s.offset;
-  if (P.load_control && s.have_last_mh) conv = conv && fabs((mh - s.last_mh) / mh) < P.thermotol;
+  if (P.load_control && s.have_last_mh) conv = conv && fabs(cq.rel_mh) < P.thermotol;
   s.last_mh = mh;
   s.have_last_mh = 1;
   const double ftol = fmax(P.forcetol, P.rel_forcetol * s.fmax);
@@ -618,6 +624,15 @@ CM_DEVINL void ccg_converge(CcgState& s, double maxdu_in, double maxpen_in) {
   } else {
     s.it += 1;
   }
+}
+
+CM_DEVINL void ccg_converge(CcgState& s, double maxdu_in, double maxpen_in) {
+  const double tf = s.total_force, mh = s.p.max_surface + s.offset;
+  ConvergeQuotients cq;
+  cq.rel_tf = (tf - (s.p.load_control ? s.p.F : s.last_tf)) / tf;
+  cq.rel_mh = (mh - s.last_mh) / mh;
+  cq.g_mean = s.G / (double)s.A_cg;
+  ccg_converge_q(s, maxdu_in, maxpen_in, cq);
 }
 
 // Row tile `tile` of the inverse pass: half spectrum -> real rows, then the

@@ -129,6 +129,26 @@ int ccg_p2_update(const CcgArgs<R>& a, cudaStream_t s, bool chained);
 template <typename R>
 int ccg_p2_ew_blocks_per_sm(const CcgArgs<R>& a);
 
+// The persistent solver of one small problem (cm_solo.cu): threads of a block,
+// the most blocks, and the length codes it serves (sides 64..1024, 96..768).
+#define CM_SOLO_THREADS 256
+#define CM_SOLO_MAX_BLOCKS 592
+#define CM_SOLO_LEN_CASES(X) X(6) X(7) X(8) X(9) X(10) X(37) X(38) X(39) X(40)
+// doubles of its partials: two buffers of CM_SOLO_NV values per block
+#define CM_SOLO_NV 12
+#define CM_SOLO_PARTIALS (2 * CM_SOLO_MAX_BLOCKS * CM_SOLO_NV)
+struct SoloPlan {
+  int grid = 0;      // blocks (0: not served)
+  int resident = 0;  // the blocks' rows of the fields stay in shared memory
+  size_t smem = 0;
+};
+template <typename R>
+SoloPlan ccg_solo_plan(const CcgArgs<R>& a, int lx, int ly);
+// Up to `iters` iterations (fewer if the solve ends); 0 when launched.
+template <typename R>
+int ccg_solo_launch(const CcgArgs<R>& a, int lx, int ly, const SoloPlan& sp, int iters,
+                    GridBarrier* bar, double* partials, cudaStream_t s);
+
 // The persistent batch kernel (cm_batch.cu): one launch over n jobs taken in
 // queue order `order` (next: a zeroed device counter), smem bytes of dynamic
 // shared memory per block; *clusters receives the clusters launched.

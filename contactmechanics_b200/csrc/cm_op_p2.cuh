@@ -224,8 +224,9 @@ k_op_row_fwd(OpArgs<R> a) {
 // Loads of one column unit k of the pair-major spectrum (rows x = 2p + b of
 // the thread's elements x = tt + q TPS, b = tt & 1): both rows of a pair load
 // Z_p(k) and Z_p(ny - k) (neighbouring lanes, one request) and each splits
-// off its own row.  Rows >= in_rows are zero.
-template <typename C, int TPS, int E>
+// off its own row.  Rows >= in_rows are zero.  CG: loads bypass L1 (a launch
+// whose other blocks write the spectrum).
+template <typename C, int TPS, int E, bool CG = false>
 CM_DEVINL void col_split_load(C (&v)[E], const C* __restrict__ spec, int ny, int k, int km, int tt,
                               int in_rows, bool ok) {
   typedef decltype(v[0].x) R;
@@ -243,8 +244,8 @@ CM_DEVINL void col_split_load(C (&v)[E], const C* __restrict__ spec, int ny, int
       z[q - h] = czero<C>();
       zm[q - h] = czero<C>();
       if (ok && x < in_rows) {
-        z[q - h] = sk[(size_t)q * pstep];
-        zm[q - h] = skm[(size_t)q * pstep];
+        z[q - h] = CG ? __ldcg(sk + (size_t)q * pstep) : sk[(size_t)q * pstep];
+        zm[q - h] = CG ? __ldcg(skm + (size_t)q * pstep) : skm[(size_t)q * pstep];
       }
     }
 #pragma unroll

@@ -31,6 +31,11 @@ struct NvtxRange {
 
 #define CM_SMEM_ROW (64 * 1024)   // ping-pong buffers of a row tile
 #define CM_COMP_ELEMS 2048
+// domain points up to which a single solve runs in the persistent kernel
+#ifndef CM_SOLO_MAX_POINTS
+#define CM_SOLO_MAX_POINTS (1u << 20)
+#endif
+#define CM_SOLO_ITERS 128  // its iterations per launch
 #define CM_MAX_PARTIAL_VALS 32
 #define CM_FP32_ITER_CAP 2000
 #define CM_FP32_ITER_CAP_PLASTIC 256
@@ -537,6 +542,8 @@ struct Work {
   int ew_grid[5] = {0, 0, 0, 0, 0};  // by-value path: grids of begin, gsum, update, bisect,
                                      // and of the one-launch bisection (0: not used)
   CcgArgs<R> ccg_args{};    // their arguments
+  SoloPlan solo;            // launch shape of the persistent solver (cm_solo.cu; grid 0: not used)
+  double* solo_partials = nullptr;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};  // [bisect passes]
   int graph_iters[2] = {0, 0};
   int graph_variant[2] = {0, 0};  // ccg_args.u_rows and fuse_gsum the graph was captured with
@@ -808,6 +815,13 @@ static int ensure_ccg(cm_plan* p, Work<R>& w) {
       const long nvec = (long)p->tx * p->ty / (16 / (long)sizeof(R));
       const long need = (nvec + 2L * 256 - 1) / (2L * 256);
       a.ew_grid = (int)std::max(1L, std::min({(long)ew_per_sm * nsm, need, (long)w.partial_blocks}));
+      if (nd <= CM_SOLO_MAX_POINTS) {
+        w.solo = ccg_solo_plan<R>(a, lx, ly);
+        if (w.solo.grid) {
+          CKS(dalloc(p, &w.solo_partials, (size_t)CM_SOLO_PARTIALS));
+          if (!w.bar) CKS(dalloc(p, &w.bar, 1));
+        }
+      }
     }
   }
   w.ccg_ready = true;
@@ -1152,11 +1166,15 @@ static int run_ccg(cm_plan* p, Work<R>& w, const cm_ccg_params* prm, const Solve
   // (set after ccg_init, whose first call on a plan initialises the arguments)
   w.ccg_args.u_rows = topo_u ? p->tx : p->nx;
   w.ccg_args.fuse_gsum = topo_u ? 1 : 0;
+  // a solve with a hardness keeps to the launched passes: its plastic mask is
+  // the sign of gaps that converge to zero, so it would change with the order
+  // of a sum
+  bool solo = w.solo.grid > 0 && prof_iters == 0 && !prm->has_hardness;
   if (w.by_value) {
     // start of the first iteration; later ones come from k_ccg_row_inv<MODE_F>
     k_ccg_begin<R><<<w.ew_grid[0], CM_THREADS, 0, s>>>(w.d_ccg, p->items, w.nt_comp);
     g_launches += 1;
-    if (w.ccg_args.fuse_gsum) {
+    if (w.ccg_args.fuse_gsum || solo) {
       CKS(ccg_p2_gsum<R>(w.ccg_args, s, true) == 0 ? CM_OK : CM_ERR_CUDA);
       g_launches += 1;
     }
@@ -1185,18 +1203,35 @@ static int run_ccg(cm_plan* p, Work<R>& w, const cm_ccg_params* prm, const Solve
   int every = prm->check_every;
   if (every <= 0) {
     const long work = (long)p->nx * p->ny;
-    every = work >= (1L << 20) ? (w.by_value ? 8 : 4) : (work >= (1L << 16) ? 8 : 16);
+    every = solo ? CM_SOLO_ITERS
+                 : work >= (1L << 20) ? (w.by_value ? 8 : 4) : (work >= (1L << 16) ? 8 : 16);
   }
   const bool observe = prm->on_iteration != nullptr && prm->iteration_forces != nullptr;
   if (observe) every = 1;
   auto t0 = std::chrono::steady_clock::now();
-  cudaGraphExec_t g;
-  CKS(get_graph<R>(p, w, bisect, every, &g));
+  cudaGraphExec_t g = nullptr;
+  if (!solo) CKS(get_graph<R>(p, w, bisect, every, &g));
+  const int lx = len_code(p->nx), ly = len_code(p->ny);
   for (int done_iters = 0;; done_iters += every) {
-    CK(cudaGraphLaunch(g, s));
-    g_launches += (unsigned long long)every *
+    if (solo) {
+      if (ccg_solo_launch<R>(w.ccg_args, lx, ly, w.solo, every, w.bar, w.solo_partials, s) == 0) {
+        g_launches += 1;
+      } else {
+        // the cooperative launch was refused (for example fewer SMs available
+        // than the occupancy query counted): the launched passes from now on
+        cudaGetLastError();
+        w.solo.grid = 0;
+        solo = false;
+        every = std::min(every, 8);
+        CKS(get_graph<R>(p, w, bisect, every, &g));
+      }
+    }
+    if (!solo) {
+      CK(cudaGraphLaunch(g, s));
+      g_launches += (unsigned long long)every *
                    (iteration_launches(bisect, w.by_value, w.by_value && w.ew_grid[4] > 0) -
                     (w.by_value && w.ccg_args.fuse_gsum ? 1 : 0));
+    }
     CK(cudaMemcpyAsync(p->h_state, w.st, sizeof(CcgState), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     ++g_polls;
