@@ -102,6 +102,37 @@ template <typename R>
 int op_p2_supported(int logx, int logy, int lw);
 template <typename R>
 int op_p2_apply(const OpArgs<R>& a, int logx, int logy, cudaStream_t s);
+
+// Transforms of any length in shared memory (cm_gen.cuh): the stages of one
+// length.
+#define CM_GEN_STAGES 12
+struct GenStage {
+  int r, Ns, m, step;  // radix, product of the radices before it, n / r, n / (Ns r)
+  FastDiv dm, dns, db; // divisions by m, by Ns, by the butterflies of a tile
+};
+struct GenFft {
+  int n = 0, nst = 0;
+  GenStage st[CM_GEN_STAGES] = {};
+};
+bool make_gen_fft(int n, GenFft* F);
+void gen_set_tile(GenFft* F, int nseq);
+int gen_row_pairs(int n, int npairs);
+template <typename R>
+int gen_col_lw(int n);
+template <typename R>
+bool gen_fits(int n);  // whether a pass of length n fits a block's shared memory
+template <typename R>
+int gen_row_fwd(const OpArgs<R>& a, GenFft F, cudaStream_t s);
+template <typename R>
+int gen_col(const OpArgs<R>& a, GenFft F, cudaStream_t s);
+template <typename R>
+int gen_row_inv(const OpArgs<R>& a, GenFft F, cudaStream_t s);
+// The operator on a domain of any sides: each axis by its register-resident
+// transforms where its length code (lx, ly) has them, else by its GenFft.
+// Same return codes as op_p2_apply.
+template <typename R>
+int op_any_apply(const OpArgs<R>& a, int lx, int ly, const GenFft& fx, const GenFft& fy,
+                 cudaStream_t s);
 // The row pass and a forward-only column pass writing the real part of the
 // 2D transform to a.fwd_real (same return codes).
 template <typename R>

@@ -328,6 +328,18 @@ int op_p2_apply(const OpArgs<R>& a, int logx, int logy, cudaStream_t s) {
 }
 
 template <typename R>
+int op_any_apply(const OpArgs<R>& a, int lx, int ly, const GenFft& fx, const GenFft& fy,
+                 cudaStream_t s) {
+  const bool px = len_ok<R>(lx), py = len_ok<R>(ly);
+  if ((!px && !gen_fits<R>(fx.n)) || (!py && !gen_fits<R>(fy.n))) return -1;
+  int rc = py ? dispatch_row_fwd<R>(ly, a, s) : gen_row_fwd<R>(a, fy, s);
+  if (!rc) rc = px ? dispatch_col<R>(lx, a, s) : gen_col<R>(a, fx, s);
+  if (!rc) rc = py ? dispatch_row_inv<R>(ly, a, s) : gen_row_inv<R>(a, fy, s);
+  if (!rc && cudaGetLastError() != cudaSuccess) rc = 1;
+  return rc;
+}
+
+template <typename R>
 int op_p2_fwd_real(const OpArgs<R>& a, int logx, int logy, cudaStream_t s) {
   if (!op_p2_supported<R>(logx, logy, a.lw) || !a.fwd_real) return -1;
   int rc = dispatch_row_fwd<R>(logy, a, s);
@@ -339,6 +351,8 @@ int op_p2_fwd_real(const OpArgs<R>& a, int logx, int logy, cudaStream_t s) {
 template int op_p2_fwd_real<double>(const OpArgs<double>&, int, int, cudaStream_t);
 template int op_p2_supported<float>(int, int, int);
 template int op_p2_supported<double>(int, int, int);
+template int op_any_apply<float>(const OpArgs<float>&, int, int, const GenFft&, const GenFft&, cudaStream_t);
+template int op_any_apply<double>(const OpArgs<double>&, int, int, const GenFft&, const GenFft&, cudaStream_t);
 template int op_p2_apply<float>(const OpArgs<float>&, int, int, cudaStream_t);
 template int op_p2_apply<double>(const OpArgs<double>&, int, int, cudaStream_t);
 template int ccg_p2_row_fwd<float, MODE_T>(const CcgArgs<float>&, int, cudaStream_t);

@@ -555,6 +555,7 @@ struct cm_plan {
   cm_plan_desc d;
   int nx, ny, nyh, tx, ty;
   FftDesc fx, fy;
+  GenFft gx, gy;  // the same lengths for the passes of cm_gen.cuh
   cudaStream_t stream;
   bool own_stream;
   double* G = nullptr;
@@ -705,7 +706,9 @@ static int init_work(cm_plan* p, Work<R>& w) {
   CKS(dalloc(p, &w.twy, p->ny));
   CK(cudaMemcpyAsync(w.twx, twx.data(), sizeof(C) * p->nx, cudaMemcpyHostToDevice, p->stream));
   CK(cudaMemcpyAsync(w.twy, twy.data(), sizeof(C) * p->ny, cudaMemcpyHostToDevice, p->stream));
-  CKS(dalloc(p, &w.spec, (size_t)p->nx * w.tiles.ntile_cols * w.tiles.col_tile));
+  // column tiles, or one row of ny per row pair (the longer for a few long rows)
+  CKS(dalloc(p, &w.spec, std::max((size_t)p->nx * w.tiles.ntile_cols * w.tiles.col_tile,
+                                  (size_t)((p->nx + 1) / 2) * p->ny)));
   CKS(dalloc(p, &w.d_plain, 1));
   CKS(dalloc(p, &w.d_ccg, 1));
   // reduction scratch is shared by the plain-operator slot and the solver
@@ -831,7 +834,7 @@ static int ensure_ccg(cm_plan* p, Work<R>& w) {
 template <typename R>
 static int launch_plain(cm_plan* p, Work<R>& w, int mode, int table_sel, const R* in, int in_rows,
                         int in_cols, int in_ld, R* out, int out_rows, int out_cols, int out_ld,
-                        cudaStream_t s) {
+                        cudaStream_t s, bool per_pass = false) {
   set_smem_attrs<R>();
   Slot<R> hs = base_slot(p, w);
   hs.in = in;
@@ -844,9 +847,11 @@ static int launch_plain(cm_plan* p, Work<R>& w, int mode, int table_sel, const R
   hs.out_ld = out_ld;
   hs.table_sel = table_sel;
   if (mode == MODE_PLAIN) {
-    // domain sides 2^k and 3 * 2^m: the by-value operator passes (cm_op_p2.cuh)
+    // the by-value operator passes: cm_op_p2.cuh along axes of 2^k and 3 * 2^m
+    // points, cm_gen.cuh along the others
     const int lx = len_code(p->nx), ly = len_code(p->ny);
-    if (lx > 0 && ly > 0 && op_p2_supported<R>(lx, ly, w.tiles.lw)) {
+    const bool p2 = lx > 0 && ly > 0 && op_p2_supported<R>(lx, ly, w.tiles.lw);
+    if (p2 || (w.tiles.generic_ok && !per_pass)) {
       OpArgs<R> a;
       a.in = in;
       a.out = out;
@@ -868,7 +873,7 @@ static int launch_plain(cm_plan* p, Work<R>& w, int mode, int table_sel, const R
       a.st = nullptr;
       a.cg_only = 0;
       a.fwd_real = nullptr;
-      const int rc = op_p2_apply<R>(a, lx, ly, s);
+      const int rc = p2 ? op_p2_apply<R>(a, lx, ly, s) : op_any_apply<R>(a, lx, ly, p->gx, p->gy, s);
       if (rc == 0) {
         g_launches += 3;
         return CM_OK;
@@ -1141,14 +1146,19 @@ static int ccg_init(cm_plan* p, Work<R>& w, const cm_ccg_params* prm, const Solv
   k_h_var<R><<<w.nt_comp, CM_THREADS, 0, s>>>(w.d_ccg, p->items, in.h64, prm->pentol <= 0, rel_pentol);
   Slot<R> hs = base_slot(p, w);
   const int gd = grid_for((long)p->nx * p->ny);
+  // a solve with a hardness runs in one arithmetic from its first field on
+  // (see run_ccg)
   if (in.f0) {
     k_init_f<R><<<gd, 256, 0, s>>>(hs, in.f0, in.f0_ld);
     CKS(launch_plain<R>(p, w, MODE_PLAIN, CM_OP_DISP, w.f[0], p->tx, p->ty, p->ty, w.u, p->nx,
-                              p->ny, p->ny, s));
+                              p->ny, p->ny, s, prm->has_hardness != 0));
   } else {
     k_init_u<R><<<gd, 256, 0, s>>>(hs, in.u0, st.p.offset0);
+    // the stiffness amplifies the shortest waves, so the first forces carry
+    // rounding that a loosely converged solve still shows: they stay with the
+    // per-pass transforms
     CKS(launch_plain<R>(p, w, MODE_PLAIN, CM_OP_FORCE, w.u, p->nx, p->ny, p->ny, w.f[0], p->tx,
-                              p->ty, p->ty, s));
+                              p->ty, p->ty, s, true));
   }
   CK(cudaGetLastError());
   return CM_OK;
@@ -1910,7 +1920,9 @@ int cm_plan_create(const cm_plan_desc* desc, void* stream, cm_plan** out) {
     cm_plan_destroy(p);
     return code;
   };
-  if (!make_fft_desc(p->nx, &p->fx) || !make_fft_desc(p->ny, &p->fy)) return fail(CM_ERR_SIZE);
+  if (!make_fft_desc(p->nx, &p->fx) || !make_fft_desc(p->ny, &p->fy) ||
+      !make_gen_fft(p->nx, &p->gx) || !make_gen_fft(p->ny, &p->gy))
+    return fail(CM_ERR_SIZE);
   if (stream) {
     p->stream = (cudaStream_t)stream;
     p->own_stream = false;
