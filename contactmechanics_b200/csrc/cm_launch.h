@@ -160,8 +160,9 @@ int ccg_p2_update(const CcgArgs<R>& a, cudaStream_t s, bool chained);
 template <typename R>
 int ccg_p2_ew_blocks_per_sm(const CcgArgs<R>& a);
 
-// The persistent solver of one small problem (cm_solo.cu): threads of a block,
-// the most blocks, and the length codes it serves (sides 64..1024, 96..768).
+// The persistent solver of one small problem (cm_solo.cuh): threads of a block,
+// the most blocks, and the length codes of its register-resident transforms
+// (sides 64..1024 and 96..768; others by cm_gen.cuh).
 #define CM_SOLO_THREADS 256
 #define CM_SOLO_MAX_BLOCKS 592
 #define CM_SOLO_LEN_CASES(X) X(6) X(7) X(8) X(9) X(10) X(37) X(38) X(39) X(40)
@@ -171,14 +172,17 @@ int ccg_p2_ew_blocks_per_sm(const CcgArgs<R>& a);
 struct SoloPlan {
   int grid = 0;      // blocks (0: not served)
   int resident = 0;  // the blocks' rows of the fields stay in shared memory
+  int elems = 0;     // transform elements of a block: its widest pass
+  int np = 0;        // row pairs of a tile (rows by cm_gen.cuh)
   size_t smem = 0;
 };
 template <typename R>
-SoloPlan ccg_solo_plan(const CcgArgs<R>& a, int lx, int ly);
+SoloPlan ccg_solo_plan(const CcgArgs<R>& a, int lx, int ly, const GenFft& gx, const GenFft& gy);
 // Up to `iters` iterations (fewer if the solve ends); 0 when launched.
 template <typename R>
-int ccg_solo_launch(const CcgArgs<R>& a, int lx, int ly, const SoloPlan& sp, int iters,
-                    GridBarrier* bar, double* partials, cudaStream_t s);
+int ccg_solo_launch(const CcgArgs<R>& a, int lx, int ly, const GenFft& gx, const GenFft& gy,
+                    const SoloPlan& sp, int iters, GridBarrier* bar, double* partials,
+                    cudaStream_t s);
 
 // The persistent batch kernel (cm_batch.cu): one launch over n jobs taken in
 // queue order `order` (next: a zeroed device counter), smem bytes of dynamic

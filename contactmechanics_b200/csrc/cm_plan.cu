@@ -818,12 +818,12 @@ static int ensure_ccg(cm_plan* p, Work<R>& w) {
       const long nvec = (long)p->tx * p->ty / (16 / (long)sizeof(R));
       const long need = (nvec + 2L * 256 - 1) / (2L * 256);
       a.ew_grid = (int)std::max(1L, std::min({(long)ew_per_sm * nsm, need, (long)w.partial_blocks}));
-      if (nd <= CM_SOLO_MAX_POINTS) {
-        w.solo = ccg_solo_plan<R>(a, lx, ly);
-        if (w.solo.grid) {
-          CKS(dalloc(p, &w.solo_partials, (size_t)CM_SOLO_PARTIALS));
-          if (!w.bar) CKS(dalloc(p, &w.bar, 1));
-        }
+    }
+    if (nd <= CM_SOLO_MAX_POINTS && w.tiles.generic_ok) {
+      w.solo = ccg_solo_plan<R>(a, lx, ly, p->gx, p->gy);
+      if (w.solo.grid) {
+        CKS(dalloc(p, &w.solo_partials, (size_t)CM_SOLO_PARTIALS));
+        if (!w.bar) CKS(dalloc(p, &w.bar, 1));
       }
     }
   }
@@ -1180,6 +1180,12 @@ static int run_ccg(cm_plan* p, Work<R>& w, const cm_ccg_params* prm, const Solve
   // the sign of gaps that converge to zero, so it would change with the order
   // of a sum
   bool solo = w.solo.grid > 0 && prof_iters == 0 && !prm->has_hardness;
+  if (solo && !w.by_value) {
+    // start of the first iteration, on the work list (sides of any length)
+    k_ccg_begin<R><<<w.nt_comp, CM_THREADS, 0, s>>>(w.d_ccg, p->items, 0);
+    k_ccg_gsum<R><<<w.nt_comp, CM_THREADS, 0, s>>>(w.d_ccg, p->items, 0);
+    g_launches += 2;
+  }
   if (w.by_value) {
     // start of the first iteration; later ones come from k_ccg_row_inv<MODE_F>
     k_ccg_begin<R><<<w.ew_grid[0], CM_THREADS, 0, s>>>(w.d_ccg, p->items, w.nt_comp);
@@ -1224,7 +1230,8 @@ static int run_ccg(cm_plan* p, Work<R>& w, const cm_ccg_params* prm, const Solve
   const int lx = len_code(p->nx), ly = len_code(p->ny);
   for (int done_iters = 0;; done_iters += every) {
     if (solo) {
-      if (ccg_solo_launch<R>(w.ccg_args, lx, ly, w.solo, every, w.bar, w.solo_partials, s) == 0) {
+      if (ccg_solo_launch<R>(w.ccg_args, lx, ly, p->gx, p->gy, w.solo, every, w.bar, w.solo_partials,
+                             s) == 0) {
         g_launches += 1;
       } else {
         // the cooperative launch was refused (for example fewer SMs available

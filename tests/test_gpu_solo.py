@@ -1,7 +1,8 @@
 """The persistent solver of small problems (cm_solo.cu) against the oracle: the
-smallest and largest sides it serves, sides 3 * 2^m, long thin domains (one
+smallest and largest sides it serves, sides 3 * 2^m, sides of any other length
+along one axis or both (odd, prime, one row pair), long thin domains (one
 pass has many tiles, the other few), free domains whose blocks hold padding
-rows only, and a domain whose blocks have several tiles each."""
+rows only, and domains whose blocks have several tiles each."""
 import numpy as np
 import pytest
 
@@ -21,6 +22,17 @@ CASES = [
     ("free", (128, 128)),
     ("free", (64, 384)),
     ("free", (256, 96)),
+    ("periodic", (75, 91)),
+    ("periodic", (64, 75)),
+    ("periodic", (75, 64)),
+    ("periodic", (96, 90)),
+    ("periodic", (67, 97)),
+    ("periodic", (20, 500)),
+    ("periodic", (1000, 30)),
+    ("periodic", (900, 700)),
+    ("free", (45, 60)),
+    ("free", (33, 32)),
+    ("free", (125, 90)),
 ]
 
 
@@ -56,7 +68,8 @@ def test_solve_fp64(kind, nb, control):
 
 
 @pytest.mark.parametrize("kind,nb", [("periodic", (64, 1024)), ("periodic", (768, 96)),
-                                     ("free", (128, 128)), ("periodic", (1024, 512))])
+                                     ("free", (128, 128)), ("periodic", (1024, 512)),
+                                     ("periodic", (75, 91)), ("free", (125, 90))])
 def test_solve_mixed(kind, nb):
     """A mixed solve meets the FP64 criteria: within the pentol of 1e-9 of the
     height range of the FP64 solution, like the other mixed tests (1e-6)."""
