@@ -23,6 +23,16 @@ def _torch():
     return torch
 
 
+def _stream_of(t):
+    """Handle of the current stream of a CUDA tensor's device, as the library
+    takes it: torch's default stream has the handle 0, which the library reads
+    as "the plan's stream", so the legacy default stream is named explicitly."""
+    torch = _torch()
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    handle = raw(t.get_device()) if raw else torch.cuda.current_stream(t.device).cuda_stream
+    return handle or _lib.CUDA_STREAM_LEGACY
+
+
 def _host(a):
     if hasattr(a, "detach") and hasattr(a, "cpu"):
         return a.detach().cpu().numpy()
@@ -226,6 +236,8 @@ class PeriodicFFTElasticHalfSpace(ElasticSubstrate):
 
     # --- operators (:573-611) ----------------------------------------------
     def _apply(self, op, field, out_shape, in_rows, in_cols, out_rows, out_cols, precision=None):
+        # On small grids a call is bound by this function, so a CUDA tensor of
+        # the operator's type passes through without torch calls of its own.
         torch = _torch()
         prec = precision or self.precision
         tdt = torch.float64 if prec == "fp64" else torch.float32
@@ -233,22 +245,19 @@ class PeriodicFFTElasticHalfSpace(ElasticSubstrate):
         if is_np:
             src = torch.from_numpy(np.ascontiguousarray(field, dtype=np.float64)).to(
                 device="cuda", dtype=tdt)
+        elif field.dtype is tdt and field.is_cuda and field.is_contiguous():
+            src = field
         else:
             src = field.to(dtype=tdt).contiguous()
             if not src.is_cuda:
                 src = src.cuda()
-        if self.dim == 1:
-            src = src.reshape(-1, 1)
-        out = torch.empty((out_rows, out_cols), dtype=tdt, device="cuda")
-        L = self._plan._L
-        # torch's default stream has the handle 0, which the library reads as
-        # "the plan's stream"; name the legacy default stream explicitly
-        stream = torch.cuda.current_stream().cuda_stream or _lib.CUDA_STREAM_LEGACY
-        _lib.check(L.cm_apply(self._plan.ptr, op, _lib.PRECISIONS[prec],
-                              ctypes.c_void_p(src.data_ptr()), in_rows, in_cols, src.shape[1],
-                              ctypes.c_void_p(out.data_ptr()), out_rows, out_cols, out_cols,
-                              ctypes.c_void_p(stream)))
-        out = out.reshape(out_shape)
+        out = torch.empty(out_shape, dtype=tdt, device="cuda")
+        # (contiguous fields: their rows are in_cols and out_cols long)
+        code = self._plan._L.cm_apply(self._plan.ptr, op, _lib.PRECISIONS[prec], src.data_ptr(),
+                                      in_rows, in_cols, in_cols, out.data_ptr(), out_rows, out_cols,
+                                      out_cols, _stream_of(out))
+        if code:
+            _lib.check(code)
         if is_np:
             return out.to(torch.float64).cpu().numpy()
         return out
