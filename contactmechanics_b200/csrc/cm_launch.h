@@ -184,6 +184,14 @@ int ccg_solo_launch(const CcgArgs<R>& a, int lx, int ly, const GenFft& gx, const
                     const SoloPlan& sp, int iters, GridBarrier* bar, double* partials,
                     cudaStream_t s);
 
+// The operator of a small domain in one cooperative launch (cm_op_one.cu).  bar
+// is the plan's own, zero before its first use; 0 when launched.
+template <typename R>
+SoloPlan op_one_plan(int nx, int ny, int lx, int ly, const GenFft& gx);
+template <typename R>
+int op_one_launch(const OpArgs<R>& a, int lx, int ly, const GenFft& gx, const SoloPlan& sp,
+                  GridBarrier* bar, cudaStream_t s);
+
 // The persistent batch kernel (cm_batch.cu): one launch over n jobs taken in
 // queue order `order` (next: a zeroed device counter), smem bytes of dynamic
 // shared memory per block; *clusters receives the clusters launched.

@@ -36,6 +36,11 @@ struct NvtxRange {
 #define CM_SOLO_MAX_POINTS (1u << 20)
 #endif
 #define CM_SOLO_ITERS 128  // its iterations per launch
+// domain points up to which the operator runs in one launch (cm_op_one.cu has
+// both sides' times)
+#ifndef CM_ONE_MAX_POINTS
+#define CM_ONE_MAX_POINTS (1L << 18)
+#endif
 #define CM_MAX_PARTIAL_VALS 32
 #define CM_FP32_ITER_CAP 2000
 #define CM_FP32_ITER_CAP_PLASTIC 256
@@ -544,6 +549,8 @@ struct Work {
   CcgArgs<R> ccg_args{};    // their arguments
   SoloPlan solo;            // launch shape of the persistent solver (cm_solo.cu; grid 0: not used)
   double* solo_partials = nullptr;
+  SoloPlan one;             // launch shape of the one-launch operator (cm_op_one.cu)
+  GridBarrier* one_bar = nullptr;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};  // [bisect passes]
   int graph_iters[2] = {0, 0};
   int graph_variant[2] = {0, 0};  // ccg_args.u_rows and fuse_gsum the graph was captured with
@@ -721,6 +728,13 @@ static int init_work(cm_plan* p, Work<R>& w) {
   CKS(dalloc(p, &w.counter, 1));
   CK(cudaMemsetAsync(w.counter, 0, sizeof(unsigned int), p->stream));
   CKS(dalloc(p, &w.st, 1));
+  if ((long)p->nx * p->ny <= CM_ONE_MAX_POINTS && w.tiles.generic_ok) {
+    w.one = op_one_plan<R>(p->nx, p->ny, len_code(p->nx), len_code(p->ny), p->gx);
+    if (w.one.grid) {
+      CKS(dalloc(p, &w.one_bar, 1));
+      CK(cudaMemsetAsync(w.one_bar, 0, sizeof(GridBarrier), p->stream));
+    }
+  }
   if (nt_max > p->max_items) p->max_items = nt_max;
   return CM_OK;
 }
@@ -873,6 +887,13 @@ static int launch_plain(cm_plan* p, Work<R>& w, int mode, int table_sel, const R
       a.st = nullptr;
       a.cg_only = 0;
       a.fwd_real = nullptr;
+      if (w.one.grid && !per_pass) {
+        if (op_one_launch<R>(a, lx, ly, p->gx, w.one, w.one_bar, s) == 0) {
+          g_launches += 1;
+          return CM_OK;
+        }
+        cudaGetLastError();  // refused (fewer SMs than counted): the launched passes
+      }
       const int rc = p2 ? op_p2_apply<R>(a, lx, ly, s) : op_any_apply<R>(a, lx, ly, p->gx, p->gy, s);
       if (rc == 0) {
         g_launches += 3;

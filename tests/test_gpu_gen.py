@@ -76,3 +76,44 @@ def test_one_dimension():
         want = oc.PeriodicSubstrate((n,), 1.0, (1.0,)).evaluate_disp(f)
         got = cm.PeriodicFFTElasticHalfSpace((n,), 1.0, (1.0,)).evaluate_disp(f)
         assert np.max(np.abs(got - want)) <= 1e-12 * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize("kind,nb", [("periodic", (64, 64)), ("periodic", (64, 1024)),
+                                     ("periodic", (1024, 64)), ("periodic", (512, 512)),
+                                     ("free", (32, 32)), ("free", (128, 64)), ("free", (64, 512))])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_one_launch_operator(kind, nb, precision):
+    """Small domains with sides 2^k (cm_op_one.cu): repeated calls and a captured
+    graph's replays leave its barrier ready for the next."""
+    import torch
+    import contactmechanics_b200 as cm
+    from contactmechanics_b200 import _lib
+    tol = 1e-12 if precision == "fp64" else 2e-5
+    f = np.random.default_rng(8).standard_normal(nb)
+    if kind == "free":
+        dom = (2 * nb[0], 2 * nb[1])
+        pad = np.zeros(dom)
+        pad[:nb[0], :nb[1]] = -f
+        want = np.fft.irfft2(np.fft.rfft2(pad) * np.fft.rfft2(oc.love_kernel_extended(nb, (1.0, 1.0), 1.0)),
+                             s=dom)[:nb[0], :nb[1]] * (nb[0] * nb[1])
+        sub = cm.FreeFFTElasticHalfSpace(nb, 1.0, (1.0, 1.0), precision=precision)
+    else:
+        want = oc.PeriodicSubstrate(nb, 1.0, (1.0, 1.0)).evaluate_disp(f)
+        sub = cm.PeriodicFFTElasticHalfSpace(nb, 1.0, (1.0, 1.0), precision=precision)
+    fd = torch.from_numpy(f).cuda().to(torch.float64 if precision == "fp64" else torch.float32)
+    n0 = _lib.lib().cm_launch_count()
+    outs = [sub.evaluate_disp(fd) for _ in range(3)]
+    assert _lib.lib().cm_launch_count() - n0 == 3
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        captured = sub.evaluate_disp(fd)
+    for _ in range(3):
+        captured.zero_()
+        graph.replay()
+        outs.append(captured.clone())
+    outs.append(sub.evaluate_disp(fd))
+    for u in outs:
+        assert np.max(np.abs(u.double().cpu().numpy() - want)) <= tol * np.max(np.abs(want))
+        assert torch.equal(u, outs[0])
