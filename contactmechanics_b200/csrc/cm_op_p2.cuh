@@ -74,6 +74,15 @@
 #define CM_COL_LW_F64 1
 #endif
 
+// Whether the column pass of type R and length code L is sized for two blocks
+// per SM.  FP64 columns of 2^11: one buffer each, so that one block's loads
+// run under the other's transforms (operator 2048^2 99.5 -> 90.8 us); of 2^10
+// there are too few blocks to pair (22.9 -> 30.9 us), and 3 * 2^m loses more by
+// the second barrier (1536^2 63.8 -> 68.9).
+#ifndef CM_COL_PAIR
+#define CM_COL_PAIR(R, L) (sizeof(R) == 8 && (L) == 11)
+#endif
+
 // log2 of the elements per thread of the solver's displacement pass
 // (k_ccg_row_inv<MODE_F>): its epilogue reads four fields per element, so it
 // keeps eight elements per thread and twice the resident warps
@@ -158,26 +167,35 @@ struct ColShape {
   static constexpr int NX = P::N;
   static constexpr int E = P::E;  // elements per thread
   static constexpr int TPS = P::TPS;
-  static constexpr size_t smem_for(int lw) {
-    return (size_t)(NX + 2 * (((NX << lw)) + ((NX << lw) >> 3) + 1)) * sizeof(C);
+  // shared memory of nbuf buffers of 2^lw columns beside the staged twiddles
+  static constexpr size_t smem_for(int lw, int nbuf) {
+    return (size_t)(NX + nbuf * (NX << lw)) * sizeof(C);
   }
-  // 32 bytes of complex values per column group, fewer if the group's
-  // ping-pong buffers do not fit
+  // 32 bytes of complex values per column group (whole sectors of the spectrum),
+  // fewer if not even one buffer of them fits
   static constexpr int LW_PREF = sizeof(C) == 8 ? CM_COL_LW_F32 : CM_COL_LW_F64;
-  static constexpr int LW = smem_for(LW_PREF) <= CM_SMEM_DYN_MAX ? LW_PREF
-                            : smem_for(LW_PREF - 1) <= CM_SMEM_DYN_MAX ? LW_PREF - 1 : 0;
+  static constexpr bool fits(int lw, int nbuf) { return smem_for(lw, nbuf) <= CM_SMEM_DYN_MAX; }
+  static constexpr bool takes(int lw) { return fits(lw, 1) && (P::TPS << lw) <= 512; }
+  static constexpr int LW = takes(LW_PREF) ? LW_PREF : takes(LW_PREF - 1) ? LW_PREF - 1 : 0;
   static constexpr int W = 1 << LW;
   static constexpr int GROUP = W * TPS;
   static constexpr int THREADS = GROUP > CM_COL_BASE ? GROUP : CM_COL_BASE;
   static constexpr int NG = THREADS / GROUP;  // column groups per block
-  static constexpr size_t BUF = (size_t)(NG * NX * W + ((NG * NX * W) >> 3) + 1) * sizeof(C);
-  // one buffer when even one column's ping-pong buffers do not fit: with the
-  // twiddles staged where they fit beside it (ONESTG: FP64 at 3 * 2^11),
-  // else read from the global table (ONEBUF: FP64 at 2^13)
-  static constexpr bool TWO = NX * sizeof(C) + 2 * BUF <= CM_SMEM_DYN_MAX;
-  static constexpr bool ONESTG = !TWO && NX * sizeof(C) + BUF <= CM_SMEM_DYN_MAX;
+  static constexpr size_t BUF = (size_t)NG * NX * W * sizeof(C);
+  // Two buffers (an exchange costs one barrier) unless one buffer (two
+  // barriers) lets two blocks share an SM or is all that fits; without room for
+  // the twiddles beside one buffer they are read from the global table (ONEBUF:
+  // FP64 at 2^13).
+  static constexpr size_t TWS = NX * sizeof(C);
+  static constexpr bool PAIRED = CM_COL_PAIR(R, LOGX);
+  static constexpr bool FIT2 = TWS + 2 * BUF <= CM_SMEM_DYN_MAX, FIT1 = TWS + BUF <= CM_SMEM_DYN_MAX;
+  static constexpr bool PAIR2 = 2 * (TWS + 2 * BUF) <= CM_SMEM_DYN_MAX, PAIR1 = 2 * (TWS + BUF) <= CM_SMEM_DYN_MAX;
+  static constexpr bool TWO = FIT2 && (PAIR2 || !PAIR1 || !PAIRED);
+  static constexpr bool ONESTG = !TWO && FIT1;
   static constexpr bool ONEBUF = !TWO && !ONESTG;
-  static constexpr size_t SMEM = TWO ? NX * sizeof(C) + 2 * BUF : ONESTG ? NX * sizeof(C) + BUF : BUF;
+  static constexpr size_t SMEM = TWO ? TWS + 2 * BUF : ONESTG ? TWS + BUF : BUF;
+  // resident blocks per SM the registers are sized for
+  static constexpr int MINB = PAIRED && 2 * SMEM <= CM_SMEM_DYN_MAX && THREADS <= 256 ? 2 : 1;
   static size_t smem() { return SMEM; }
 };
 
@@ -284,7 +302,7 @@ CM_DEVINL void col_pack_store(const C (&v)[E], C* __restrict__ spec, int ny, int
 }
 
 template <typename R, int LOGX>
-__global__ void __launch_bounds__(ColShape<R, LOGX>::THREADS, 1)
+__global__ void __launch_bounds__(ColShape<R, LOGX>::THREADS, ColShape<R, LOGX>::MINB)
 k_op_col(OpArgs<R> a) {
   typedef typename CT<R>::C C;
   typedef ColShape<R, LOGX> Sh;
@@ -293,7 +311,7 @@ k_op_col(OpArgs<R> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* tws = reinterpret_cast<C*>(smem_raw);
   C* bufA = Sh::ONEBUF ? tws : tws + NX;
-  C* bufB = bufA + smem_padded(Sh::NG * NX * W);
+  C* bufB = bufA + Sh::NG * NX * W;
   pdl_trigger();
   const C* tw = stage_twiddles<LOGX, Sh::LR, Sh::THREADS, Sh::ONEBUF>(tws, a.twx);
   pdl_wait();
