@@ -114,6 +114,10 @@
 #define CM_T3_ROW_BASE 256
 #endif
 
+#ifndef CM_ROW_AHEAD
+#define CM_ROW_AHEAD 11
+#endif
+
 // default log2 elements per thread (per part) of the row passes for length
 // code L (cm_fft_p2.cuh): FP64 transforms of length 2^13 take 16 elements
 // per thread (512 threads a sequence)
@@ -152,6 +156,9 @@ struct OpShape {
   // holds more than half of the shared memory
   static constexpr int MINB = SMEM > CM_SMEM_DYN_MAX / 2 ? 1
                               : sizeof(R) == 8 ? CM_FP64_ROW_MINB : CM_ROW_F32_MINB;
+  // whether the operator's row passes load the next tile's elements before they
+  // transform the present one (registers of the loads in flight)
+  static constexpr bool AHEAD = sizeof(R) == 8 && E <= 8 && P::F == 1 && LOGN >= CM_ROW_AHEAD;
   static size_t smem() { return SMEM; }
 };
 
@@ -216,9 +223,8 @@ k_op_row_fwd(OpArgs<R> a) {
   __syncthreads();
   const int s = threadIdx.x >> P::LTPS, tt = threadIdx.x & (P::TPS - 1);
   const int npairs = (a.in_rows + 1) >> 1;
-  for (int p0 = blockIdx.x * NP; p0 < npairs; p0 += gridDim.x * NP) {
-    const int p = p0 + s, xa = 2 * p;
-    C v[Sh::E];
+  auto load = [&](C (&v)[Sh::E], int p) {
+    const int xa = 2 * p;
 #pragma unroll
     for (int q = 0; q < Sh::E; ++q) {
       const int y = tt + q * P::TPS;
@@ -228,6 +234,19 @@ k_op_row_fwd(OpArgs<R> a) {
         if (xa + 1 < a.in_rows) rb = __ldg(a.in + (size_t)(xa + 1) * a.in_ld + y);
       }
       v[q] = cmake<C>(ra, rb);
+    }
+  };
+  C ahead[Sh::E];
+  if (Sh::AHEAD) load(ahead, blockIdx.x * NP + s);
+  for (int p0 = blockIdx.x * NP; p0 < npairs; p0 += gridDim.x * NP) {
+    const int p = p0 + s;
+    C v[Sh::E];
+    if (Sh::AHEAD) {
+#pragma unroll
+      for (int q = 0; q < Sh::E; ++q) v[q] = ahead[q];
+      load(ahead, p + gridDim.x * NP);
+    } else {
+      load(v, p);
     }
     fft_len<C, false, LOGN, Sh::LR, Sh::ONEBUF, Sh::ONESTG>(v, bufA, bufB, s * N, 1, tt, tw);
     if (p < npairs) {
@@ -374,12 +393,23 @@ k_op_row_inv(OpArgs<R> a) {
   __syncthreads();
   const int s = threadIdx.x >> P::LTPS, tt = threadIdx.x & (P::TPS - 1);
   const int npairs = (a.out_rows + 1) >> 1;
-  for (int p0 = blockIdx.x * NP; p0 < npairs; p0 += gridDim.x * NP) {
-    const int p = p0 + s, xa = 2 * p;
-    C v[Sh::E];
+  auto load = [&](C (&v)[Sh::E], int p) {
     const C* __restrict__ row = a.spec + (size_t)p * N;
 #pragma unroll
     for (int q = 0; q < Sh::E; ++q) v[q] = p < npairs ? row[kfreq<LOGN, Sh::LR>(tt, q)] : czero<C>();
+  };
+  C ahead[Sh::E];
+  if (Sh::AHEAD) load(ahead, blockIdx.x * NP + s);
+  for (int p0 = blockIdx.x * NP; p0 < npairs; p0 += gridDim.x * NP) {
+    const int p = p0 + s, xa = 2 * p;
+    C v[Sh::E];
+    if (Sh::AHEAD) {
+#pragma unroll
+      for (int q = 0; q < Sh::E; ++q) v[q] = ahead[q];
+      load(ahead, p + gridDim.x * NP);
+    } else {
+      load(v, p);
+    }
     fft_len<C, true, LOGN, Sh::LR, Sh::ONEBUF, Sh::ONESTG>(v, bufA, bufB, s * N, 1, tt, tw);
 #pragma unroll
     for (int q = 0; q < Sh::E; ++q) {
