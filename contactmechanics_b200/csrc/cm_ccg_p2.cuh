@@ -253,7 +253,7 @@ k_ccg_row_inv(CcgArgs<R> a) {
   R du = 0, pmax = -INFINITY;                     // MODE_F: extrema, exact in R
   R gmax = -INFINITY, gmin = INFINITY;
   int n_c = 0, n_cg = 0;                          // counts, exact in int
-  double s_cg = 0, s_cg2 = 0;                     // sums of g and g^2 over the CG area
+  double s_cg = 0, s1 = 0, s2 = 0;                // sums of g, g - off and (g - off)^2 over the CG area
   const R* __restrict__ fn_buf = a.f[cv.par ^ 1];
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int x0 = tile * ROWS;
@@ -358,10 +358,17 @@ k_ccg_row_inv(CcgArgs<R> a) {
             n_c += c0;
             n_cg += c;
             if (c) s_cg += (double)g;
-            // the reference sums c g^2 over the whole topography, so a NaN
-            // gap outside the contact set makes G NaN as well
-            if (c) s_cg2 += (double)g * (double)g;
-            else if (isnan(g)) s_cg2 += (double)g;
+            if (a.fuse_gsum) {
+              // the reference sums c g^2 over the whole topography, so a NaN
+              // gap outside the contact set makes G NaN as well
+              const double gs = (double)g - cv.offset;
+              if (c) {
+                s1 += gs;
+                s2 += gs * gs;
+              } else if (isnan(g)) {
+                s2 += (double)g;
+              }
+            }
             gmax = fmax(gmax, g);
             gmin = fmin(gmin, g);
           }
@@ -376,23 +383,26 @@ k_ccg_row_inv(CcgArgs<R> a) {
     tile_finish<1>(st, a.partials, a.counter, blockIdx.x, gridDim.x, vr, kinds,
                    [&](CcgState& s, double (&r)[1]) { fin_tau(s, r); });
   } else {
-    double vr[8] = {(double)du, (double)pmax, (double)n_c, (double)n_cg, s_cg, (double)gmax,
-                    (double)gmin, s_cg2};
+    // both counts in one value: each is at most 2^26
+    constexpr double PACK = 134217728.0;
+    double vr[8] = {(double)du, (double)pmax, (double)n_c + PACK * (double)n_cg, s1, s_cg,
+                    (double)gmax, (double)gmin, s2};
     const int kinds[8] = {RED_MAX, RED_MAX, RED_SUM, RED_SUM, RED_SUM, RED_MAX, RED_MIN, RED_SUM};
     const int fuse = a.fuse_gsum;
+    const double off64 = cv.offset;
     tile_finish<8>(st, a.partials, a.counter, blockIdx.x, gridDim.x, vr, kinds,
                    [&](CcgState& s, double (&r)[8]) {
       ccg_converge(s, r[0], r[1]);
       if (!s.done) {
-        double b[5] = {r[2], r[3], r[4], r[5], r[6]};
+        const double cg = floor(r[2] / PACK);
+        double b[5] = {r[2] - PACK * cg, cg, r[4], r[5], r[6]};
         fin_begin(s, b);
         if (fuse && s.branch == 0) {
-          // G = sum over c of (g - offset)^2 from the sums over c of g^2
-          // and g (each g^2 of an FP32 gap is exact in FP64); near
-          // convergence this loses about eps64 * sum g^2 / G, far below the
-          // FP32 gaps' own rounding
-          const double off = s.offset;
-          double G = r[7] - 2.0 * off * r[4] + (double)s.A_cg * off * off;
+          // G = sum over c of (g - offset)^2 from the sums S1, S2 of the gaps
+          // from this iteration's offset: it cancels only as far as the offset
+          // moves against the residual within one iteration
+          const double d = s.offset - off64;
+          double G = r[7] - 2.0 * d * r[3] + (double)s.A_cg * d * d;
           if (G < 0) G = 0;  // rounding (a NaN stays NaN)
           double gv[1] = {G};
           fin_gsum(s, gv);

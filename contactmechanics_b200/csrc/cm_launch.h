@@ -63,9 +63,9 @@ struct CcgArgs {
                  // FP32 phase of a mixed solve (the padding's displacement
                  // feeds only max |du| and the result, which the FP64 phase
                  // recomputes from the forces)
-  int fuse_gsum; // the displacement pass also forms the next iteration's G
-                 // (FP32 phase of a mixed solve; the iterations then run
-                 // without the gsum pass)
+  int fuse_gsum; // the displacement pass also forms the next iteration's G (the
+                 // iterations then run without the gsum pass); not with a
+                 // hardness, whose plastic mask would change with its rounding
   FastDiv ew_vpr;  // 16-byte vectors per topography row (element-wise passes)
 };
 // Launch with programmatic stream serialization: the kernel may start while

@@ -1193,10 +1193,9 @@ static int run_ccg(cm_plan* p, Work<R>& w, const cm_ccg_params* prm, const Solve
   cudaStream_t s = p->stream;
   CKS(ccg_init(p, w, prm, in, rel_pentol, rel_forcetol, maxiter, s));
   // topo_u (FP32 phase of a mixed solve): the displacement pass updates
-  // the topography's rows only and forms the next iteration's G as well
-  // (set after ccg_init, whose first call on a plan initialises the arguments)
+  // the topography's rows only (set after ccg_init, whose first call on a plan initialises the arguments)
   w.ccg_args.u_rows = topo_u ? p->tx : p->nx;
-  w.ccg_args.fuse_gsum = topo_u ? 1 : 0;
+  w.ccg_args.fuse_gsum = (topo_u || !prm->has_hardness) ? 1 : 0;
   // a solve with a hardness keeps to the launched passes: its plastic mask is
   // the sign of gaps that converge to zero, so it would change with the order
   // of a sum
