@@ -35,7 +35,6 @@ k_ccg_row_fwd(CcgArgs<R> a) {
   C* tws = reinterpret_cast<C*>(smem_raw);
   C* bufA = Sh::ONEBUF ? tws : tws + N;
   C* bufB = bufA + smem_padded(NP * N);
-  pdl_trigger();
   if (threadIdx.x == 0) {
     mbar_init(&mbar, 1);
     mbar_init_fence();
@@ -198,6 +197,7 @@ k_ccg_row_fwd(CcgArgs<R> a) {
     }
     __syncthreads();  // buffers free for the next tile
   }
+  pdl_trigger();
   if (MODE == MODE_T) {
     double vr[1] = {acc};
     const int kinds[1] = {RED_SUM};
@@ -229,7 +229,6 @@ k_ccg_row_inv(CcgArgs<R> a) {
   C* tws = reinterpret_cast<C*>(smem_raw);
   C* bufA = Sh::ONEBUF ? tws : tws + N;
   C* bufB = bufA + smem_padded(NP * N);
-  pdl_trigger();
   const C* tw = stage_twiddles<LOGN, Sh::LR, Sh::THREADS, Sh::ONEBUF>(tws, a.op.twy);
   pdl_wait();
   CcgState* st = a.st;
@@ -377,6 +376,7 @@ k_ccg_row_inv(CcgArgs<R> a) {
     }
     __syncthreads();  // buffers free for the next tile
   }
+  pdl_trigger();
   if (MODE == MODE_T) {
     double vr[1] = {a0};
     const int kinds[1] = {RED_SUM};
@@ -475,7 +475,6 @@ __global__ void __launch_bounds__(CM_EW_THREADS) k_ew_gsum(CcgArgs<R> a) {
   constexpr int V = VR::V;
   const EwIndex<P2> ix = ew_index<P2>(a);
   const long nvec = (long)a.tx * a.ty / V;
-  pdl_trigger();
   pdl_wait();
   CcgState* st = a.st;
   CcgView cv;
@@ -516,6 +515,7 @@ __global__ void __launch_bounds__(CM_EW_THREADS) k_ew_gsum(CcgArgs<R> a) {
       }
     }
   }
+  pdl_trigger();
   double v[1] = {G};
   const int kinds[1] = {RED_SUM};
   tile_finish<1>(st, a.partials, a.counter, blockIdx.x, gridDim.x, v, kinds,
@@ -530,7 +530,6 @@ __global__ void __launch_bounds__(CM_EW_THREADS) k_ew_update(CcgArgs<R> a) {
   constexpr int V = VR::V;
   const EwIndex<P2> ix = ew_index<P2>(a);
   const long nvec = (long)a.tx * a.ty / V;
-  pdl_trigger();
   pdl_wait();
   CcgState* st = a.st;
   CcgView cv;
@@ -606,6 +605,7 @@ __global__ void __launch_bounds__(CM_EW_THREADS) k_ew_update(CcgArgs<R> a) {
       }
     }
   }
+  pdl_trigger();
   double v[5] = {(double)a_fl, (double)min_fn + H, (double)max_t, s_fp, (double)n_nc};
   const int kinds[5] = {RED_SUM, RED_MIN, RED_MAX, RED_SUM, RED_SUM};
   tile_finish<5>(st, a.partials, a.counter, blockIdx.x, gridDim.x, v, kinds,

@@ -58,7 +58,10 @@ template <typename C, typename R> CM_DEVINL C cmake(R x, R y) { C r; r.x = x; r.
 // room); pdl_wait blocks until every preceding grid the launch depends on has
 // completed and its memory is visible.  A kernel launched without the
 // programmatic-serialization attribute was already ordered behind its
-// predecessor, and both are no-ops for it.  Kernels read only constant
+// predecessor, and both are no-ops for it.  The passes of a solve trigger when
+// a block has done its tiles: triggered at their start, a whole iteration of
+// waiting kernels takes their places early and slows the running one (free
+// 1024^2 FP64 solve 23.1 ms, 22.4 with plain launches, 22.25 so).  Kernels read only constant
 // inputs (twiddle tables, launch arguments) before pdl_wait.
 CM_DEVINL void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 CM_DEVINL void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

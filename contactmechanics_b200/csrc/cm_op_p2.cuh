@@ -331,7 +331,6 @@ k_op_col(OpArgs<R> a) {
   C* tws = reinterpret_cast<C*>(smem_raw);
   C* bufA = Sh::ONEBUF ? tws : tws + NX;
   C* bufB = bufA + Sh::NG * NX * W;
-  pdl_trigger();
   const C* tw = stage_twiddles<LOGX, Sh::LR, Sh::THREADS, Sh::ONEBUF>(tws, a.twx);
   pdl_wait();
   if (a.st && (a.st->done || (a.cg_only && a.st->branch != 0))) return;
@@ -374,6 +373,7 @@ k_op_col(OpArgs<R> a) {
     col_pack_store<C, P::TPS, W, E>(v, a.spec, ny, k, km, tt, a.out_rows, ok);
     __syncthreads();  // buffers free for the next group
   }
+  pdl_trigger();
 }
 
 template <typename R, int LOGN>
