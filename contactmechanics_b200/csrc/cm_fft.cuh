@@ -13,13 +13,16 @@
 #pragma once
 #include "cm_common.cuh"
 
-#define CM_MAX_STAGES 24
+#define CM_MAX_STAGES 9  // lengths that fit shared memory (below 16384) have at most 8
 
 struct FftDesc {
   int n;
   int nst;
   int generic;  // 1 when a stage radix is outside {2,3,4,5,7,8}
   int rad[CM_MAX_STAGES];
+  // divisions by n / radix and by the product of the radices before a stage
+  // (three integer divisions a butterfly cost as much as a radix-4 one)
+  FastDiv dm[CM_MAX_STAGES], dns[CM_MAX_STAGES];
 };
 
 // twiddle lookup (the table is staged in shared memory by the caller)
@@ -109,16 +112,16 @@ struct Dft<INV, 8, C> {
 // thread walks its butterflies one at a time, so only RR values are live.
 template <typename C, bool INV, int RR>
 CM_DEVINL void fft_stage(const C* src, C* dst, int n, int Ns, int nseq, int sstride, int estride,
-                         bool seq_fastest, const C* tw) {
-  const int m = n / RR;
+                         int lw, FastDiv dm, FastDiv dns, const C* tw) {
+  const int m = dm.d;
   const int B = m * nseq;
-  const int step = n / (Ns * RR);
+  const int step = fdiv(dns, m);
   for (int bi = threadIdx.x; bi < B; bi += blockDim.x) {
     int s, j;
-    if (seq_fastest) { s = bi % nseq; j = bi / nseq; }
-    else { j = bi % m; s = bi / m; }
+    if (lw >= 0) { s = bi & ((1 << lw) - 1); j = bi >> lw; }
+    else { s = fdiv(dm, bi); j = bi - s * m; }
     const C* in = src + s * sstride;
-    const int k = j % Ns;
+    const int k = j - fdiv(dns, j) * Ns;
     C v[RR];
 #pragma unroll
     for (int q = 0; q < RR; ++q) v[q] = in[(j + q * m) * estride];
@@ -140,19 +143,19 @@ CM_DEVINL void fft_stage(const C* src, C* dst, int n, int Ns, int nseq, int sstr
 // Direct DFT stage for an arbitrary radix r (prime factors above 7).
 template <typename C, bool INV>
 CM_DEVINL void fft_stage_generic(const C* src, C* dst, int n, int r, int Ns, int nseq,
-                                 int sstride, int estride, bool seq_fastest,
+                                 int sstride, int estride, int lw, FastDiv dm, FastDiv dns,
                                  const C* tw) {
-  const int m = n / r;
+  const int m = dm.d;
   const int B = m * nseq;
-  const int step = n / (Ns * r);
-  const int ws = n / r;
+  const int step = fdiv(dns, m);
+  const int ws = m;
   for (int bi = threadIdx.x; bi < B; bi += blockDim.x) {
     int s, j;
-    if (seq_fastest) { s = bi % nseq; j = bi / nseq; }
-    else { j = bi % m; s = bi / m; }
+    if (lw >= 0) { s = bi & ((1 << lw) - 1); j = bi >> lw; }
+    else { s = fdiv(dm, bi); j = bi - s * m; }
     const C* in = src + s * sstride;
     C* out = dst + s * sstride;
-    const int k = j % Ns;
+    const int k = j - fdiv(dns, j) * Ns;
     const int ob = (j - k) * r + k;
     for (int q = 0; q < r; ++q) {
       C acc = czero<C>();
@@ -172,21 +175,23 @@ CM_DEVINL void fft_stage_generic(const C* src, C* dst, int n, int r, int Ns, int
 }
 
 // Transform all sequences; data starts in `a`, `b` is a buffer of the same
-// size.  Returns the buffer that holds the result.
+// size.  Returns the buffer that holds the result.  lw >= 0: 2^lw sequences
+// whose index runs fastest over the threads (column tiles), else whole
+// sequences one after the other.
 template <typename C, bool INV>
 CM_DEVINL C* fft_smem(C* a, C* b, const FftDesc& d, int nseq, int sstride, int estride,
-                      bool seq_fastest, const C* tw) {
+                      int lw, const C* tw) {
   int Ns = 1;
   for (int st = 0; st < d.nst; ++st) {
     const int r = d.rad[st];
     switch (r) {
-      case 8: fft_stage<C, INV, 8>(a, b, d.n, Ns, nseq, sstride, estride, seq_fastest, tw); break;
-      case 4: fft_stage<C, INV, 4>(a, b, d.n, Ns, nseq, sstride, estride, seq_fastest, tw); break;
-      case 2: fft_stage<C, INV, 2>(a, b, d.n, Ns, nseq, sstride, estride, seq_fastest, tw); break;
-      case 3: fft_stage<C, INV, 3>(a, b, d.n, Ns, nseq, sstride, estride, seq_fastest, tw); break;
-      case 5: fft_stage<C, INV, 5>(a, b, d.n, Ns, nseq, sstride, estride, seq_fastest, tw); break;
-      case 7: fft_stage<C, INV, 7>(a, b, d.n, Ns, nseq, sstride, estride, seq_fastest, tw); break;
-      default: fft_stage_generic<C, INV>(a, b, d.n, r, Ns, nseq, sstride, estride, seq_fastest, tw); break;
+      case 8: fft_stage<C, INV, 8>(a, b, d.n, Ns, nseq, sstride, estride, lw, d.dm[st], d.dns[st], tw); break;
+      case 4: fft_stage<C, INV, 4>(a, b, d.n, Ns, nseq, sstride, estride, lw, d.dm[st], d.dns[st], tw); break;
+      case 2: fft_stage<C, INV, 2>(a, b, d.n, Ns, nseq, sstride, estride, lw, d.dm[st], d.dns[st], tw); break;
+      case 3: fft_stage<C, INV, 3>(a, b, d.n, Ns, nseq, sstride, estride, lw, d.dm[st], d.dns[st], tw); break;
+      case 5: fft_stage<C, INV, 5>(a, b, d.n, Ns, nseq, sstride, estride, lw, d.dm[st], d.dns[st], tw); break;
+      case 7: fft_stage<C, INV, 7>(a, b, d.n, Ns, nseq, sstride, estride, lw, d.dm[st], d.dns[st], tw); break;
+      default: fft_stage_generic<C, INV>(a, b, d.n, r, Ns, nseq, sstride, estride, lw, d.dm[st], d.dns[st], tw); break;
     }
     C* t = a;
     a = b;

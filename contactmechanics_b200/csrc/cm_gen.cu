@@ -134,10 +134,11 @@ const RadixPlan& plan_radices(int n, std::map<int, RadixPlan>& memo) {
 // Big direct stages first (no twiddles on their inputs), then odd radices (a
 // stage writes runs of as many elements as the stages before it covered, so
 // the first strides should share no factor with the banks), then even ones.
-bool make_gen_fft(int n, GenFft* F) {
+void make_gen_fft(int n, GenFft* F) {
   std::map<int, RadixPlan> memo;
   std::vector<int> rad = plan_radices(n, memo).rad;
-  if ((int)rad.size() > CM_GEN_STAGES) return false;
+  // (only lengths beyond any pass have more)
+  if ((int)rad.size() > CM_GEN_STAGES) rad.resize(CM_GEN_STAGES);
   std::sort(rad.begin(), rad.end(), [](int a, int b) {
     const bool ba = a > 16 || a == 11 || a == 13, bb = b > 16 || b == 11 || b == 13;
     if (ba != bb) return ba;
@@ -159,7 +160,6 @@ bool make_gen_fft(int n, GenFft* F) {
     S.db = make_fastdiv(1);  // set per launch: butterflies of a tile
     Ns *= rad[i];
   }
-  return true;
 }
 
 // butterflies of a tile of nseq sequences, for the direct stages' item index

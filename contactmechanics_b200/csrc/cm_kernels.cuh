@@ -393,22 +393,23 @@ CM_DEVINL void row_fwd_tile(const Slot<R>* __restrict__ Sp, const CcgView& cv, i
     R* __restrict__ t = Sp->t;
     const R off = (R)cv.offset;
     struct In { R f[2], u[2], h[2], t[2]; };
+    // loads from addresses that are valid without a test (the row's first
+    // element for columns beyond the topography, the tile's first row for a
+    // missing one), so that the loads of a round are all in flight together
     batched_loop<2>(npairs * ny, [&](int e) {
-      const int p = fdiv(dny, e), y = e - p * ny;
+      const int p = fdiv(dny, e), y = e - p * ny, yy = y < ty ? y : 0;
       In v;
 #pragma unroll
       for (int w = 0; w < 2; ++w) {
-        const int x = x0 + 2 * p + w;
-        v.f[w] = 0; v.u[w] = 0; v.h[w] = 0; v.t[w] = 0;
-        if (x < x0 + nrows && y < ty) {
-          const size_t ic = (size_t)x * ty + y;
-          v.f[w] = ldf(fio + ic);
-          if (MODE == MODE_T || cv.apply_nc) {
-            v.u[w] = ldf(u + (size_t)x * ny + y);
-            v.h[w] = ldf(h + ic);
-          }
-          if (MODE == MODE_T) v.t[w] = ldf(t + ic);
+        const int xw = x0 + 2 * p + w, x = xw < x0 + nrows ? xw : x0;
+        const size_t ic = (size_t)x * ty + yy;
+        v.f[w] = ldf(fio + ic);
+        v.u[w] = 0; v.h[w] = 0; v.t[w] = 0;
+        if (MODE == MODE_T || cv.apply_nc) {
+          v.u[w] = ldf(u + (size_t)x * ny + yy);
+          v.h[w] = ldf(h + ic);
         }
+        if (MODE == MODE_T) v.t[w] = ldf(t + ic);
       }
       return v;
     }, [&](int e, const In& v) {
@@ -452,7 +453,7 @@ CM_DEVINL void row_fwd_tile(const Slot<R>* __restrict__ Sp, const CcgView& cv, i
     });
   }
   __syncthreads();
-  const C* res = fft_smem<C, false>(buf, scratch, fd, npairs, ny, 1, false, tws);
+  const C* res = fft_smem<C, false>(buf, scratch, fd, npairs, ny, 1, -1, tws);
   for (int e = threadIdx.x; e < npairs * nyh; e += blockDim.x) {
     const int p = fdiv(dnyh, e), k = e - p * nyh;
     const C z = res[p * ny + k];
@@ -524,34 +525,20 @@ CM_DEVINL void col_tile(const Slot<R>* __restrict__ Sp, int tile, const FftDesc&
   // the tile is one contiguous block of nx * W elements in HBM
   C* __restrict__ blk = Sp->spec + (size_t)tile * nx * W;
   const R* __restrict__ tblk = tab + (size_t)tile * nx * W;
-  const int total = nx * wc;
-  if (wc == W) {
-    batched_loop<8>(nx_in * W, [&](int e) { return ldf(blk + e); }, [&](int e, C v) { buf[e] = v; });
-    for (int e = nx_in * W + threadIdx.x; e < total; e += blockDim.x) buf[e] = czero<C>();
-  } else {
-    batched_loop<8>(total, [&](int e) {
-      const int x = e / wc, c = e - x * wc;
-      return (x < nx_in) ? ldf(blk + x * W + c) : czero<C>();
-    }, [&](int e, C v) { buf[e] = v; });
-  }
+  // (a last tile of fewer columns is padded with zeros to W)
+  batched_loop<8>(nx_in * W, [&](int e) { return (e & (W - 1)) < wc ? ldf(blk + e) : czero<C>(); },
+                  [&](int e, C v) { buf[e] = v; });
+  for (int e = nx_in * W + threadIdx.x; e < nx * W; e += blockDim.x) buf[e] = czero<C>();
   __syncthreads();
-  C* res = fft_smem<C, false>(buf, scratch, fd, wc, 1, wc, true, tws);
+  C* res = fft_smem<C, false>(buf, scratch, fd, W, 1, W, lw, tws);
   if (MODE != MODE_FWD) {
-    batched_loop<8>(total, [&](int e) {
-      const int x = e / wc, c = e - x * wc;
-      return __ldg(tblk + x * W + c);
-    }, [&](int e, R g) { res[e] = cscale(res[e], g); });
+    batched_loop<8>(nx * W, [&](int e) { return (e & (W - 1)) < wc ? __ldg(tblk + e) : (R)0; },
+                    [&](int e, R g) { res[e] = cscale(res[e], g); });
     __syncthreads();
-    res = fft_smem<C, true>(res, res == buf ? scratch : buf, fd, wc, 1, wc, true, tws);
+    res = fft_smem<C, true>(res, res == buf ? scratch : buf, fd, W, 1, W, lw, tws);
   }
-  if (wc == W) {
-    for (int e = threadIdx.x; e < nx_out * W; e += blockDim.x) blk[e] = res[e];
-  } else {
-    for (int e = threadIdx.x; e < nx_out * wc; e += blockDim.x) {
-      const int x = e / wc, c = e - x * wc;
-      blk[x * W + c] = res[e];
-    }
-  }
+  for (int e = threadIdx.x; e < nx_out * W; e += blockDim.x)
+    if ((e & (W - 1)) < wc) blk[e] = res[e];
 }
 
 template <typename R, int MODE>
@@ -638,12 +625,18 @@ CM_DEVINL void ccg_converge(CcgState& s, double maxdu_in, double maxpen_in) {
 // Row tile `tile` of the inverse pass: half spectrum -> real rows, then the
 // caller's buffer, or the CCG epilogue.  fd / tws / buf / scratch as for
 // row_fwd_tile.  a0 / a1 collect this thread's share of the tile's sums
-// (MODE_T: sum r t; MODE_F: max |du|, max penetration over the CG set).
+// (MODE_T: sum r t; MODE_F: max |du|, max penetration over the CG set).  fuse
+// (MODE_F): nx_it collects the next iteration's start of an elastic solve, from
+// the new displacement and the iteration's final force.
+struct NextIter {
+  int n_c = 0;                     // contact points
+  double s_cg = 0, s1 = 0, s2 = 0; // sums over them of g, g - off, (g - off)^2
+};
 template <typename R, int MODE>
 CM_DEVINL void row_inv_tile(const Slot<R>* __restrict__ Sp, const CcgView& cv, int tile,
                             const FftDesc& fd, const typename CT<R>::C* tws,
                             typename CT<R>::C* buf, typename CT<R>::C* scratch, double& a0,
-                            double& a1) {
+                            double& a1, NextIter& nx_it, bool fuse) {
   typedef typename CT<R>::C C;
   const int nx = Sp->nx, ny = Sp->ny, nyh = Sp->nyh, ty = Sp->ty, tx = Sp->tx, lw = Sp->lw;
   const int rows_total = (MODE == MODE_PLAIN) ? Sp->out_rows : (MODE == MODE_T ? tx : nx);
@@ -670,7 +663,7 @@ CM_DEVINL void row_inv_tile(const Slot<R>* __restrict__ Sp, const CcgView& cv, i
     if (!selfconj) buf[p * ny + ny - k] = cmake<C>(X.x + Y.y, Y.x - X.y);
   });
   __syncthreads();
-  const C* res = fft_smem<C, true>(buf, scratch, fd, npairs, ny, 1, false, tws);
+  const C* res = fft_smem<C, true>(buf, scratch, fd, npairs, ny, 1, -1, tws);
   if (MODE == MODE_PLAIN) {
     R* __restrict__ out = Sp->out;
     const int out_cols = Sp->out_cols, out_ld = Sp->out_ld;
@@ -702,23 +695,25 @@ CM_DEVINL void row_inv_tile(const Slot<R>* __restrict__ Sp, const CcgView& cv, i
     R* __restrict__ u = Sp->u;
     const R* __restrict__ h = Sp->h;
     const R* __restrict__ fa_buf = Sp->f[cv.par];
+    const R* __restrict__ fn_buf = Sp->f[cv.par ^ 1];
     const unsigned char* __restrict__ gneg = Sp->gneg;
     const R off = (R)cv.offset;
-    struct UF { R uo[2], fa[2], h[2]; unsigned char gn[2]; };
-    batched_loop<2>(npairs * ny, [&](int e) {
-      const int p = fdiv(dny, e), y = e - p * ny;
+    struct UF { R uo[2], fa[2], h[2], fn[2]; unsigned char gn[2]; };
+    const bool topo = x0 < tx;  // else a tile of padding rows
+    batched_loop<sizeof(R) == 8 ? 1 : 2>(npairs * ny, [&](int e) {
+      const int p = fdiv(dny, e), y = e - p * ny, yy = y < ty ? y : 0;
       UF v;
 #pragma unroll
       for (int w = 0; w < 2; ++w) {
-        const int x = x0 + 2 * p + w;
-        v.uo[w] = 0; v.fa[w] = 0; v.h[w] = 0; v.gn[w] = 0;
-        if (x >= x0 + nrows) continue;
+        const int xw = x0 + 2 * p + w, x = xw < x0 + nrows ? xw : x0;
         v.uo[w] = ldf(u + (size_t)x * ny + y);
-        if (x < tx && y < ty) {
-          const size_t ic = (size_t)x * ty + y;
+        v.fa[w] = 0; v.h[w] = 0; v.fn[w] = 0; v.gn[w] = 0;
+        if (topo) {
+          const size_t ic = (size_t)(x < tx ? x : x0) * ty + yy;
           v.h[w] = ldf(h + ic);
           if (cv.branch == 0) v.fa[w] = ldf(fa_buf + ic);
           else v.gn[w] = ldf(gneg + ic);
+          if (fuse) v.fn[w] = ldf(fn_buf + ic);
         }
       }
       return v;
@@ -738,6 +733,20 @@ CM_DEVINL void row_inv_tile(const Slot<R>* __restrict__ Sp, const CcgView& cv, i
           else c = v.gn[w] != 0;
           const R pen = (v.h[w] + off) - val;
           a1 = fmax(a1, c ? (double)pen : 0.0);
+          if (fuse) {
+            const R g = val - v.h[w];
+            // the reference sums c g^2 over the whole topography, so a NaN gap
+            // outside the contact set makes G NaN as well
+            if (v.fn[w] < 0) {
+              const double gs = (double)g - cv.offset;
+              nx_it.n_c += 1;
+              nx_it.s_cg += (double)g;
+              nx_it.s1 += gs;
+              nx_it.s2 += gs * gs;
+            } else if (isnan(g)) {
+              nx_it.s2 += (double)g;
+            }
+          }
         }
       }
     });
@@ -764,12 +773,32 @@ k_row_inv(const Slot<R>* __restrict__ slots, const int2* __restrict__ items) {
   C* scratch = buf + (Sp->row_tile >> 1) * ny;
   stage_fft(fd, Sp->fy, tws, Sp->twy, ny);
   double a0 = 0.0, a1 = -INFINITY;  // MODE_T: sum r t ; MODE_F: max|du|, max penetration
-  row_inv_tile<R, MODE>(Sp, cv, item.y, fd, tws, buf, scratch, a0, a1);
+  NextIter next;
+  const bool fuse = MODE == MODE_F && Sp->fuse;
+  row_inv_tile<R, MODE>(Sp, cv, item.y, fd, tws, buf, scratch, a0, a1, next, fuse);
   if (MODE == MODE_T) {
     double v[1] = {a0};
     const int kinds[1] = {RED_SUM};
     tile_finish<1>(st, Sp->partials, Sp->counter, item.y, Sp->nt_rowt, v, kinds,
                    [&](CcgState& s, double (&a)[1]) { fin_tau(s, a); });
+  } else if (MODE == MODE_F && fuse) {
+    double v[6] = {a0, a1, (double)next.n_c, next.s_cg, next.s1, next.s2};
+    const int kinds[6] = {RED_MAX, RED_MAX, RED_SUM, RED_SUM, RED_SUM, RED_SUM};
+    const double off64 = cv.offset;
+    tile_finish<6>(st, Sp->partials, Sp->counter, item.y, Sp->nt_rowd, v, kinds,
+                   [&](CcgState& s, double (&a)[6]) {
+      ccg_converge(s, a[0], a[1]);
+      if (!s.done) {
+        double b[5] = {a[2], a[2], a[3], 0.0, 0.0};
+        fin_begin(s, b);
+        // G from the sums of the gaps measured from this iteration's offset
+        const double d = s.offset - off64;
+        double G = a[5] - 2.0 * d * a[4] + a[2] * d * d;
+        if (G < 0) G = 0;  // rounding (a NaN stays NaN)
+        double gv[1] = {G};
+        fin_gsum(s, gv);
+      }
+    });
   } else if (MODE == MODE_F) {
     double v[2] = {a0, a1};
     const int kinds[2] = {RED_MAX, RED_MAX};
@@ -810,7 +839,9 @@ struct CompTile {
 // solves share a launch) and writes one partial per tile.  With strided = n
 // > 0 every item is a tile of the one solve of items[0], the block walks
 // tiles blockIdx.x, blockIdx.x + gridDim.x, ... < n and writes one partial
-// for all of them (fewer blocks and partials for a single solve).
+// for all of them (fewer blocks and partials for a single solve).  The begin and
+// gsum passes skip solves whose displacement pass does their work (Slot::fuse),
+// but for strided = -1, the first iteration's start of those solves alone.
 struct EwTiles {
   int first, end, step, part, nparts;
   CM_DEVINL EwTiles(int2 item, int strided, int nt_comp) {
@@ -854,6 +885,7 @@ __global__ void __launch_bounds__(CM_THREADS)
 k_ccg_begin(const Slot<R>* __restrict__ slots, const int2* __restrict__ items, int strided) {
   const int2 item = items[strided > 0 ? 0 : blockIdx.x];
   const Slot<R>* __restrict__ Sp = slots + item.x;
+  if (strided <= 0 && (Sp->fuse != 0) != (strided < 0)) return;
   CcgState* st = Sp->st;
   // the slot (geometry, field pointers) is constant during a solve: read it
   // before waiting for the previous kernel
@@ -903,6 +935,7 @@ __global__ void __launch_bounds__(CM_THREADS)
 k_ccg_gsum(const Slot<R>* __restrict__ slots, const int2* __restrict__ items, int strided) {
   const int2 item = items[strided > 0 ? 0 : blockIdx.x];
   const Slot<R>* __restrict__ Sp = slots + item.x;
+  if (strided <= 0 && (Sp->fuse != 0) != (strided < 0)) return;
   CcgState* st = Sp->st;
   const EwTiles W(item, strided, Sp->nt_comp);
   R* const f0 = Sp->f[0];

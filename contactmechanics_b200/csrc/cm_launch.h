@@ -114,7 +114,7 @@ struct GenFft {
   int n = 0, nst = 0;
   GenStage st[CM_GEN_STAGES] = {};
 };
-bool make_gen_fft(int n, GenFft* F);
+void make_gen_fft(int n, GenFft* F);
 void gen_set_tile(GenFft* F, int nseq);
 int gen_row_pairs(int n, int npairs);
 template <typename R>

@@ -94,9 +94,10 @@ static bool make_fft_desc(int n, FftDesc* d) {
   memset(d, 0, sizeof(*d));
   d->n = n;
   int m = n, k = 0;
+  // (longer lengths, whose transforms no pass holds, may run out of stages;
+  // they keep their tables only)
   auto push = [&](int r) {
-    if (k >= CM_MAX_STAGES) return false;
-    d->rad[k++] = r;
+    if (k < CM_MAX_STAGES) d->rad[k++] = r;
     return true;
   };
   while (m % 8 == 0 && m >= 8) { if (!push(8)) return false; m /= 8; }
@@ -113,6 +114,12 @@ static bool make_fft_desc(int n, FftDesc* d) {
     }
   }
   d->nst = k;
+  int Ns = 1;
+  for (int i = 0; i < k; ++i) {
+    d->dm[i] = make_fastdiv((unsigned)(n / d->rad[i]));
+    d->dns[i] = make_fastdiv((unsigned)Ns);
+    Ns *= d->rad[i];
+  }
   return true;
 }
 
@@ -1396,6 +1403,7 @@ struct BatchDev {
   int n_items[4] = {0, 0, 0, 0};
   int* running = nullptr;  // count of running solves, then one done flag per solve
   size_t smem_row = 0, smem_col = 0;
+  bool fuse = false;  // Slot::fuse of every slot
   std::vector<void*> allocs;
   ~BatchDev() {
     for (void* a : allocs) cudaFree(a);
@@ -1460,11 +1468,13 @@ template <typename R>
 static void launch_iteration_batch(const BatchDev<R>& b, bool bisect, cudaStream_t s) {
   const Slot<R>* S = b.slots;
   const int TT = g_batch_threads[sizeof(R) == 8 ? 0 : 1];  // threads of the transform launches
-  k_ccg_begin<R><<<b.n_items[0], CM_THREADS, 0, s>>>(S, b.items[0], 0);
-  if (bisect)
-    for (int i = 0; i < CM_BISECT_PASSES; ++i)
-      k_ccg_bisect<R><<<b.n_items[0], CM_THREADS, 0, s>>>(S, b.items[0], 0);
-  k_ccg_gsum<R><<<b.n_items[0], CM_THREADS, 0, s>>>(S, b.items[0], 0);
+  if (!b.fuse) {
+    k_ccg_begin<R><<<b.n_items[0], CM_THREADS, 0, s>>>(S, b.items[0], 0);
+    if (bisect)
+      for (int i = 0; i < CM_BISECT_PASSES; ++i)
+        k_ccg_bisect<R><<<b.n_items[0], CM_THREADS, 0, s>>>(S, b.items[0], 0);
+    k_ccg_gsum<R><<<b.n_items[0], CM_THREADS, 0, s>>>(S, b.items[0], 0);
+  }
   k_row_fwd<R, MODE_T><<<b.n_items[1], TT, b.smem_row, s>>>(S, b.items[1]);
   k_col<R, MODE_T><<<b.n_items[3], TT, b.smem_col, s>>>(S, b.items[3]);
   k_row_inv<R, MODE_T><<<b.n_items[1], TT, b.smem_row, s>>>(S, b.items[1]);
@@ -1525,7 +1535,7 @@ static int batch_loop(int n, cm_plan* const* plans, BatchDev<R>& b, bool bisect,
   auto t0 = std::chrono::steady_clock::now();
   for (int done_iters = 0; running > 0; done_iters += every) {
     if (cudaGraphLaunch(ge, s) != cudaSuccess) { rc = CM_ERR_CUDA; break; }
-    g_launches += (unsigned long long)every * (iteration_launches(bisect, false)) + 1;
+    g_launches += (unsigned long long)every * (iteration_launches(bisect, false) - (b.fuse ? 2 : 0)) + 1;
     if (cudaMemcpyAsync(flags.data(), b.running, sizeof(int) * (1 + n), cudaMemcpyDeviceToHost, s) !=
             cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess) { rc = CM_ERR_CUDA; break; }
@@ -1568,8 +1578,11 @@ static int lockstep_phase(int n, cm_plan* const* plans, const cm_ccg_params* par
   set_smem_attrs<R>();
   for (int i = 0; i < n; ++i) CKS(ensure_ccg(plans[i], work_of<R>(plans[i])));
   BatchDev<R> b;
+  b.fuse = true;
+  for (int i = 0; i < n; ++i) b.fuse = b.fuse && !params[i].has_hardness;
   CKS(batch_build<R>(n, plans, b, s, [&](int i, Slot<R>& sl) {
     cm_plan* p = plans[i];
+    sl.fuse = !params[i].has_hardness;
     sl.h64 = h[i];
     sl.u0 = (!from_fp32 && u0) ? u0[i] : nullptr;
     sl.prev_f[0] = p->w32.f[0];
@@ -1623,6 +1636,11 @@ static int lockstep_phase(int n, cm_plan* const* plans, const cm_ccg_params* par
     k_row_inv<R, MODE_PLAIN><<<b.n_items[2], TT, b.smem_row, s>>>(S, b.items[2]);
   }
   g_launches += 7;
+  // the first iteration's start of the solves without a hardness (later ones
+  // come from the displacement pass)
+  k_ccg_begin<R><<<b.n_items[0], CM_THREADS, 0, s>>>(S, b.items[0], -1);
+  k_ccg_gsum<R><<<b.n_items[0], CM_THREADS, 0, s>>>(S, b.items[0], -1);
+  g_launches += 2;
   CK(cudaGetLastError());
   CKS(batch_loop<R>(n, plans, b, bisect, maxiter_all, timeout, s, polls));
   if (final) {
@@ -1947,9 +1965,9 @@ int cm_plan_create(const cm_plan_desc* desc, void* stream, cm_plan** out) {
     cm_plan_destroy(p);
     return code;
   };
-  if (!make_fft_desc(p->nx, &p->fx) || !make_fft_desc(p->ny, &p->fy) ||
-      !make_gen_fft(p->nx, &p->gx) || !make_gen_fft(p->ny, &p->gy))
-    return fail(CM_ERR_SIZE);
+  if (!make_fft_desc(p->nx, &p->fx) || !make_fft_desc(p->ny, &p->fy)) return fail(CM_ERR_SIZE);
+  make_gen_fft(p->nx, &p->gx);
+  make_gen_fft(p->ny, &p->gy);
   if (stream) {
     p->stream = (cudaStream_t)stream;
     p->own_stream = false;

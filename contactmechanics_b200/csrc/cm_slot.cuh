@@ -106,6 +106,8 @@ struct Slot {
   CcgState* st;
   double* partials;
   unsigned int* counter;
+  int fuse;  // the displacement pass also starts the next iteration (batches
+             // without a hardness; the begin and gsum passes then run only once)
   // lockstep batches: per-solve inputs and results of the batched set-up
   // and result kernels (unused elsewhere)
   const double* h64;        // FP64 heights (tx, ty)
