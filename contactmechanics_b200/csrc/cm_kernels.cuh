@@ -465,8 +465,14 @@ CM_DEVINL void row_fwd_tile(const Slot<R>* __restrict__ Sp, const CcgView& cv, i
   }
 }
 
+// Registers of the FP64 transform passes: three 256-thread blocks per SM (the
+// 64-solve batch's row passes 70 -> 66, 62 -> 57, 56 -> 49 us, columns 45 -> 39),
+// but for the displacement pass, whose epilogue spills there (121 -> 129).
+template <typename R, int MODE, bool INV>
+constexpr int pass_regs() { return sizeof(R) == 8 && !(INV && MODE == MODE_F) ? 80 : 128; }
+
 template <typename R, int MODE>
-__global__ void __launch_bounds__(CM_FFT_THREADS)
+__global__ void __maxnreg__((pass_regs<R, MODE, false>()))
 k_row_fwd(const Slot<R>* __restrict__ slots, const int2* __restrict__ items) {
   typedef typename CT<R>::C C;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -542,7 +548,7 @@ CM_DEVINL void col_tile(const Slot<R>* __restrict__ Sp, int tile, const FftDesc&
 }
 
 template <typename R, int MODE>
-__global__ void __launch_bounds__(CM_FFT_THREADS)
+__global__ void __maxnreg__((pass_regs<R, MODE, false>()))
 k_col(const Slot<R>* __restrict__ slots, const int2* __restrict__ items) {
   typedef typename CT<R>::C C;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -754,7 +760,7 @@ CM_DEVINL void row_inv_tile(const Slot<R>* __restrict__ Sp, const CcgView& cv, i
 }
 
 template <typename R, int MODE>
-__global__ void __launch_bounds__(CM_FFT_THREADS)
+__global__ void __maxnreg__((pass_regs<R, MODE, true>()))
 k_row_inv(const Slot<R>* __restrict__ slots, const int2* __restrict__ items) {
   typedef typename CT<R>::C C;
   extern __shared__ __align__(16) unsigned char smem_raw[];

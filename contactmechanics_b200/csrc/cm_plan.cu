@@ -1513,7 +1513,10 @@ static int batch_loop(int n, cm_plan* const* plans, BatchDev<R>& b, bool bisect,
                       double timeout_s, cudaStream_t s, int* polls) {
   long work = 0;
   for (int i = 0; i < n; ++i) work += (long)plans[i]->nx * plans[i]->ny;
-  const int every = work >= (1L << 22) ? 4 : 16;
+  // iterations between polls: a poll costs about 15 us and the iterations a
+  // group runs past the last convergence are wasted (64 solves of sides 64..512:
+  // 300-430 us each, 6 of 48 and 32 on average in groups of 16)
+  const int every = work >= (1L << 20) ? 4 : work >= (1L << 17) ? 8 : 16;
   cudaGraphExec_t ge = nullptr;
   auto capture = [&]() -> int {
     if (ge) cudaGraphExecDestroy(ge);
