@@ -16,7 +16,12 @@
 // multiply-adds a butterfly spread over r / 4 threads, the root's index kept
 // by addition.  (Recomputing twiddled inputs and (p q) mod r inside a double
 // loop on one thread per butterfly, the 73-point stages of a 511 x 256
-// domain took 534 us a column pass.)
+// domain took 534 us a column pass; here 12.)
+//
+// Operator FP64, mixed-radix passes / these: 500 x 300 49.2 / 22.6 us, 1000^2
+// 63.6 / 50, 167^2 2750 / 33, 511 x 256 565 / 20.5.  Bound by the stages'
+// latency on small grids: radices up to 5, 6 or 9 only gave the same times up to
+// 500^2 and lost at 1000^2 (47 -> 58-63).
 #pragma once
 #include "cm_fft_p2.cuh"
 #include "cm_kernels.cuh"

@@ -68,12 +68,12 @@ int row_fwd(const OpArgs<R>& a, cudaStream_t s, bool launch = true) {
   if constexpr (!len_fits<R, LOGN>()) {
     return -1;
   } else {
-    typedef OpShape<R, LOGN> Sh;
+    typedef OpRowShape<R, LOGN> Sh;
     static KernelInfo info;
     int rc;
     {
       std::lock_guard<std::mutex> g(g_op_mu);
-      rc = prepare<R, LOGN>(k_op_row_fwd<R, LOGN>, info);
+      rc = prepare<R, LOGN, decltype(&k_op_row_fwd<R, LOGN>), Sh>(k_op_row_fwd<R, LOGN>, info);
     }
     if (rc || !launch) return rc;
     const int tiles = (a.in_rows + 2 * Sh::NP - 1) / (2 * Sh::NP);
@@ -83,14 +83,14 @@ int row_fwd(const OpArgs<R>& a, cudaStream_t s, bool launch = true) {
   }
 }
 
-template <typename R, int LOGX, typename K>
-int prepare_col(K kernel, KernelInfo& info) {
-  typedef ColShape<R, LOGX> Sh;
+template <typename R, int LOGX, int BASE>
+int prepare_col(KernelInfo& info) {
+  typedef ColShape<R, LOGX, BASE> Sh;
   if (info.ready) return info.grid_per_sm > 0 ? 0 : -1;
   const size_t smem = Sh::smem();
   if (smem > CM_SMEM_DYN_MAX) return -1;
-  if (cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess)
+  const void* kernel = (const void*)k_op_col<R, LOGX, BASE>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return 1;
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, Sh::THREADS, smem) != cudaSuccess)
@@ -100,27 +100,38 @@ int prepare_col(K kernel, KernelInfo& info) {
   return per_sm > 0 ? 0 : -1;
 }
 
-// column pass on the pair-major spectrum (k_op_col); LOGX: log2 of the
-// column length (domain rows)
+template <typename R, int LOGX, int BASE>
+int col_base(const OpArgs<R>& a, int groups, cudaStream_t s, bool launch) {
+  typedef ColShape<R, LOGX, BASE> Sh;
+  static KernelInfo info;
+  int rc;
+  {
+    std::lock_guard<std::mutex> g(g_op_mu);
+    rc = prepare_col<R, LOGX, BASE>(info);
+  }
+  if (rc || !launch) return rc;
+  const int blocks = (groups + Sh::NG - 1) / Sh::NG;
+  const int grid = std::max(1, std::min(blocks, info.grid_per_sm * sm_count()));
+  launch_pdl(k_op_col<R, LOGX, BASE>, grid, Sh::THREADS, Sh::smem(), s, a);
+  return 0;
+}
+
+// column pass on the pair-major spectrum (k_op_col); LOGX: length code of the
+// columns (domain rows).  Short columns of a small grid, and of sides 3 * 2^m,
+// take small blocks (CM_COL_BASE_SHORT).
 template <typename R, int LOGX>
 int col(const OpArgs<R>& a, cudaStream_t s, bool launch = true) {
   if constexpr (!len_fits<R, LOGX>()) {
     return -1;
   } else {
     typedef ColShape<R, LOGX> Sh;
-    static KernelInfo info;
-    int rc;
-    {
-      std::lock_guard<std::mutex> g(g_op_mu);
-      rc = prepare_col<R, LOGX>(k_op_col<R, LOGX>, info);
-    }
-    if (rc || !launch) return rc;
     const int units = a.ny / 2 + 1;
     const int groups = (units + Sh::W - 1) / Sh::W;
-    const int blocks = (groups + Sh::NG - 1) / Sh::NG;
-    const int grid = std::max(1, std::min(blocks, info.grid_per_sm * sm_count()));
-    launch_pdl(k_op_col<R, LOGX>, grid, Sh::THREADS, Sh::smem(), s, a);
-    return 0;
+    if constexpr (Sh::NG > 1) {
+      if (LOGX >= 32 || 2 * ((groups + Sh::NG - 1) / Sh::NG) <= sm_count())
+        return col_base<R, LOGX, CM_COL_BASE_SHORT>(a, groups, s, launch);
+    }
+    return col_base<R, LOGX, CM_COL_BASE>(a, groups, s, launch);
   }
 }
 
@@ -129,12 +140,12 @@ int row_inv(const OpArgs<R>& a, cudaStream_t s, bool launch = true) {
   if constexpr (!len_fits<R, LOGN>()) {
     return -1;
   } else {
-    typedef OpShape<R, LOGN> Sh;
+    typedef OpRowShape<R, LOGN> Sh;
     static KernelInfo info;
     int rc;
     {
       std::lock_guard<std::mutex> g(g_op_mu);
-      rc = prepare<R, LOGN>(k_op_row_inv<R, LOGN>, info);
+      rc = prepare<R, LOGN, decltype(&k_op_row_inv<R, LOGN>), Sh>(k_op_row_inv<R, LOGN>, info);
     }
     if (rc || !launch) return rc;
     const int tiles = (a.out_rows + 2 * Sh::NP - 1) / (2 * Sh::NP);

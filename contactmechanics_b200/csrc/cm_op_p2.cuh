@@ -57,6 +57,15 @@
 #define CM_COL_BASE 256
 #endif
 
+// ... for a grid with too few columns to give every second SM such a block (512^2
+// FP64: 33 blocks of 256 threads, 129 of 64; plastic 512^2 solve 9.3 -> 8.5 ms,
+// operator FP64 384^2 21.6 -> 15.0 us).  With more columns the larger blocks
+// stage fewer twiddles (512 x 2048 24.9 us, 26.9 with blocks of 64); columns of
+// 3 * 2^m points keep to the small ones (768 x 1536 FP64 41.0 -> 39.2 us).
+#ifndef CM_COL_BASE_SHORT
+#define CM_COL_BASE_SHORT 64
+#endif
+
 // log2 of the elements per thread of the column pass's transforms
 #ifndef CM_COL_LR_F32
 #define CM_COL_LR_F32 4
@@ -114,6 +123,10 @@
 #define CM_T3_ROW_BASE 256
 #endif
 
+// log2 of the FP64 rows from which the operator's row passes load the next tile
+// before they transform the present one: with one or two blocks per SM nothing
+// else runs under the loads (operator FP64 4096^2 393 -> 369 us, 2048^2 90.5 ->
+// 88.4); shorter rows have a tile or two per block (1024^2 22.9 -> 23.3)
 #ifndef CM_ROW_AHEAD
 #define CM_ROW_AHEAD 11
 #endif
@@ -133,7 +146,7 @@ constexpr int row_lr(int code) {
 // staged twiddles do not fit a block's shared memory (FP64 at 2^13), so the
 // transform runs on one buffer with the twiddles read from global memory;
 // ONESTG: one buffer and the staged twiddles fit (FP64 at 3 * 2^11).
-template <typename R, int LOGN, int LRV = row_lr<R>(LOGN)>
+template <typename R, int LOGN, int LRV = row_lr<R>(LOGN), int SHORT = 0>
 struct OpShape {
   typedef typename CT<R>::C C;
   typedef FftLen<LOGN, LRV> P;
@@ -141,7 +154,9 @@ struct OpShape {
   static constexpr int LR = LRV;
   static constexpr int E = P::E;  // elements per thread
   static constexpr int TPS = P::TPS;
-  static constexpr int BASE = P::F == 3 ? CM_T3_ROW_BASE
+  // (SHORT: threads of a block for rows of up to 512 points)
+  static constexpr int BASE = SHORT && N <= 512 ? SHORT
+                              : P::F == 3 ? CM_T3_ROW_BASE
                                         : (sizeof(R) == 8 ? 256 : CM_ROW_F32_BASE) >> (LR - 3);
   static constexpr int THREADS = TPS > BASE ? TPS : BASE;
   static constexpr int NP = THREADS / TPS;  // row pairs per block
@@ -165,7 +180,7 @@ struct OpShape {
 // Column pass for columns of length code LOGX: 16 elements per thread for
 // 2^LOGX (3 x 2^LR for 3 * 2^m), groups of W = 2^LW columns with the column
 // index fastest across threads.
-template <typename R, int LOGX>
+template <typename R, int LOGX, int BASE = CM_COL_BASE>
 struct ColShape {
   typedef typename CT<R>::C C;
   static constexpr int LR = LenCode<LOGX>::F == 3 ? (sizeof(R) == 8 ? CM_T3_LR_F64 : CM_T3_LR_F32)
@@ -186,7 +201,7 @@ struct ColShape {
   static constexpr int LW = takes(LW_PREF) ? LW_PREF : takes(LW_PREF - 1) ? LW_PREF - 1 : 0;
   static constexpr int W = 1 << LW;
   static constexpr int GROUP = W * TPS;
-  static constexpr int THREADS = GROUP > CM_COL_BASE ? GROUP : CM_COL_BASE;
+  static constexpr int THREADS = GROUP > BASE ? GROUP : BASE;
   static constexpr int NG = THREADS / GROUP;  // column groups per block
   static constexpr size_t BUF = (size_t)NG * NX * W * sizeof(C);
   // Two buffers (an exchange costs one barrier) unless one buffer (two
@@ -206,11 +221,17 @@ struct ColShape {
   static size_t smem() { return SMEM; }
 };
 
+// the operator's own row passes: small blocks on short rows, for the same
+// reason as CM_COL_BASE_SHORT (a solve's row passes keep theirs, the order of
+// their sums with it)
 template <typename R, int LOGN>
-__global__ void __launch_bounds__(OpShape<R, LOGN>::THREADS, OpShape<R, LOGN>::MINB)
+using OpRowShape = OpShape<R, LOGN, row_lr<R>(LOGN), 64>;
+
+template <typename R, int LOGN>
+__global__ void __launch_bounds__(OpRowShape<R, LOGN>::THREADS, OpRowShape<R, LOGN>::MINB)
 k_op_row_fwd(OpArgs<R> a) {
   typedef typename CT<R>::C C;
-  typedef OpShape<R, LOGN> Sh;
+  typedef OpRowShape<R, LOGN> Sh;
   typedef typename Sh::P P;
   constexpr int N = P::N, NP = Sh::NP;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -320,17 +341,18 @@ CM_DEVINL void col_pack_store(const C (&v)[E], C* __restrict__ spec, int ny, int
   }
 }
 
-template <typename R, int LOGX>
-__global__ void __launch_bounds__(ColShape<R, LOGX>::THREADS, ColShape<R, LOGX>::MINB)
+template <typename R, int LOGX, int BASE = CM_COL_BASE>
+__global__ void __launch_bounds__(ColShape<R, LOGX, BASE>::THREADS, ColShape<R, LOGX, BASE>::MINB)
 k_op_col(OpArgs<R> a) {
   typedef typename CT<R>::C C;
-  typedef ColShape<R, LOGX> Sh;
+  typedef ColShape<R, LOGX, BASE> Sh;
   typedef typename Sh::P P;
   constexpr int NX = P::N, W = Sh::W, LW = Sh::LW, E = Sh::E;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* tws = reinterpret_cast<C*>(smem_raw);
   C* bufA = Sh::ONEBUF ? tws : tws + NX;
   C* bufB = bufA + Sh::NG * NX * W;
+  if (!a.st) pdl_trigger();  // (one call's inverse rows; a solve's launches follow its tiles)
   const C* tw = stage_twiddles<LOGX, Sh::LR, Sh::THREADS, Sh::ONEBUF>(tws, a.twx);
   pdl_wait();
   if (a.st && (a.st->done || (a.cg_only && a.st->branch != 0))) return;
@@ -373,14 +395,14 @@ k_op_col(OpArgs<R> a) {
     col_pack_store<C, P::TPS, W, E>(v, a.spec, ny, k, km, tt, a.out_rows, ok);
     __syncthreads();  // buffers free for the next group
   }
-  pdl_trigger();
+  if (a.st) pdl_trigger();
 }
 
 template <typename R, int LOGN>
-__global__ void __launch_bounds__(OpShape<R, LOGN>::THREADS, OpShape<R, LOGN>::MINB)
+__global__ void __launch_bounds__(OpRowShape<R, LOGN>::THREADS, OpRowShape<R, LOGN>::MINB)
 k_op_row_inv(OpArgs<R> a) {
   typedef typename CT<R>::C C;
-  typedef OpShape<R, LOGN> Sh;
+  typedef OpRowShape<R, LOGN> Sh;
   typedef typename Sh::P P;
   constexpr int N = P::N, NP = Sh::NP;
   extern __shared__ __align__(16) unsigned char smem_raw[];

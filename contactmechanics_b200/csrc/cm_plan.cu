@@ -31,11 +31,14 @@ struct NvtxRange {
 
 #define CM_SMEM_ROW (64 * 1024)   // ping-pong buffers of a row tile
 #define CM_COMP_ELEMS 2048
-// domain points up to which a single solve runs in the persistent kernel
+// domain points up to which a single solve without a hardness runs in the
+// persistent kernel (cm_solo.cuh has both sides' times)
 #ifndef CM_SOLO_MAX_POINTS
 #define CM_SOLO_MAX_POINTS (1u << 20)
 #endif
-#define CM_SOLO_ITERS 128  // its iterations per launch
+// its iterations per launch: a solve of a few tens ends in one, and other streams' work
+// waits a few milliseconds at most
+#define CM_SOLO_ITERS 64
 // domain points up to which the operator runs in one launch (cm_op_one.cu has
 // both sides' times)
 #ifndef CM_ONE_MAX_POINTS
@@ -840,13 +843,6 @@ static int ensure_ccg(cm_plan* p, Work<R>& w) {
       const long need = (nvec + 2L * 256 - 1) / (2L * 256);
       a.ew_grid = (int)std::max(1L, std::min({(long)ew_per_sm * nsm, need, (long)w.partial_blocks}));
     }
-    if (nd <= CM_SOLO_MAX_POINTS && w.tiles.generic_ok) {
-      w.solo = ccg_solo_plan<R>(a, lx, ly, p->gx, p->gy);
-      if (w.solo.grid) {
-        CKS(dalloc(p, &w.solo_partials, (size_t)CM_SOLO_PARTIALS));
-        if (!w.bar) CKS(dalloc(p, &w.bar, 1));
-      }
-    }
   }
   w.ccg_ready = true;
   return CM_OK;
@@ -1206,7 +1202,18 @@ static int run_ccg(cm_plan* p, Work<R>& w, const cm_ccg_params* prm, const Solve
   // a solve with a hardness keeps to the launched passes: its plastic mask is
   // the sign of gaps that converge to zero, so it would change with the order
   // of a sum
-  bool solo = w.solo.grid > 0 && prof_iters == 0 && !prm->has_hardness;
+  bool solo = prof_iters == 0 && !prm->has_hardness && w.tiles.generic_ok &&
+              (size_t)p->nx * p->ny <= CM_SOLO_MAX_POINTS;
+  if (solo && !w.solo_partials) {
+    // the plan's first solve of this kind (batches never need these)
+    // (its launch shape for the whole domain's rows, whatever this phase updates)
+    CcgArgs<R> whole = w.ccg_args;
+    whole.u_rows = p->nx;
+    w.solo = ccg_solo_plan<R>(whole, len_code(p->nx), len_code(p->ny), p->gx, p->gy);
+    CKS(dalloc(p, &w.solo_partials, (size_t)CM_SOLO_PARTIALS));
+    if (!w.bar) CKS(dalloc(p, &w.bar, 1));
+  }
+  solo = solo && w.solo.grid > 0;
   if (solo && !w.by_value) {
     // start of the first iteration, on the work list (sides of any length)
     k_ccg_begin<R><<<w.nt_comp, CM_THREADS, 0, s>>>(w.d_ccg, p->items, 0);

@@ -6,7 +6,7 @@
 // solve's state, and ends with a ticket that one last block turns into the
 // next scalar (periodic 256^2 FP64: seven passes of 5-10 us, of which the
 // transforms take 1.3 us each).  Here the blocks stay, the twiddles stay in shared
-// memory, and the passes are separated by a grid barrier (about 1 us).
+// memory, and the passes are separated by a grid barrier (1.2-1.5 us).
 //
 //   rows forward of t | columns | rows inverse, sum r t | force update |
 //   rows forward of f | columns | rows inverse, u, next iteration's start
@@ -30,6 +30,18 @@
 //   sums of the gaps measured from the present offset, off:
 //   G = S2 - 2 d S1 + A d^2, d = new offset - off, which cancels only as far
 //   as the offset moves against the residual within one iteration.
+//
+// What bounds it: the chain of barriers (2400-2900 cycles each on 33-148 blocks,
+// the same for flags per block and for arrivals per warp) and of a few warps'
+// instruction latencies.  So four elements per thread (eight took 34 us an
+// iteration of periodic 256^2 FP64, four 30), one loop body for both operators
+// (with every pass written out and unrolled the iteration's code left the
+// instruction cache: 48 us), poll and abort in one load, and the divisions of
+// the convergence step side by side.  Per iteration, launched passes / here,
+// FP64: periodic 64^2 68 / 30 us, 256^2 76 / 31, 512^2 89 / 34, 768^2 96 / 61,
+// 1024^2 95 / 79, free 128^2 77 / 33, 512^2 81 / 61; mixed alike.  Beyond 2^20
+// domain points every SM has many tiles and the launched passes' larger
+// butterflies win.
 //
 // Waits are bounded (CM_BARRIER_TIMEOUT_CYCLES): a block that gives up raises
 // the abort word, every other wait sees it, and the solve ends with

@@ -179,8 +179,8 @@ int cm_plan_shape(const cm_plan* plan, int* nxd, int* nyd, int* nyh);
 /*
  * Which transform engine serves the plan's operator and single solves in
  * `precision` (CM_FP64 or CM_FP32): *engine = 1 for the register-resident
- * passes (domain sides 2^k and 3 * 2^m), 0 for the shared-memory
- * mixed-radix passes of every other size.  No counterpart in the reference
+ * passes (domain sides 2^k and 3 * 2^m), 0 where at least one side takes the
+ * shared-memory transforms of any length.  No counterpart in the reference
  * (numpy's FFT serves every size there).
  */
 int cm_plan_engine(const cm_plan* plan, int precision, int* engine);

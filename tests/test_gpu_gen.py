@@ -117,3 +117,27 @@ def test_one_launch_operator(kind, nb, precision):
     for u in outs:
         assert np.max(np.abs(u.double().cpu().numpy() - want)) <= tol * np.max(np.abs(want))
         assert torch.equal(u, outs[0])
+
+
+@pytest.mark.parametrize("nb", [(64, 64), (45, 60), (2048, 64)])
+def test_input_forms(nb):
+    """Transposed, strided, other types, host tensors and arrays give what a
+    contiguous CUDA tensor of the operator's type gives."""
+    import torch
+    import contactmechanics_b200 as cm
+    sub = cm.PeriodicFFTElasticHalfSpace(nb, 1.0, (1.0, 1.0))
+    f = torch.from_numpy(np.random.default_rng(9).standard_normal(nb)).cuda()
+    f = f.float().double()  # values that both types hold
+    want = sub.evaluate_disp(f)
+    strided = torch.zeros((nb[0], 2 * nb[1]), dtype=f.dtype, device="cuda")
+    strided[:, ::2] = f
+    for g in (f.t().contiguous().t(), strided[:, ::2], f.float(), f.cpu()):
+        assert torch.equal(sub.evaluate_disp(g), want)
+    assert np.array_equal(sub.evaluate_disp(f.cpu().numpy()), want.cpu().numpy())
+    assert np.array_equal(sub.evaluate_disp(np.asfortranarray(f.cpu().numpy())), want.cpu().numpy())
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        again = sub.evaluate_disp(f)
+    torch.cuda.current_stream().wait_stream(side)
+    assert torch.equal(again, want)
