@@ -27,8 +27,8 @@
 // runs on the per-pass path) and without a wall-clock timeout.
 //
 // Measured on a B200 against the lockstep graph of per-pass launches (the
-// default batch path): 331 ms against 294 ms for 512 mixed-precision solves
-// of sides 64..512, 31 ms against 25 ms for 36.  With every body of the
+// default batch path): 287 ms against 174 ms for 512 mixed-precision solves
+// of sides 64..512.  With every body of the
 // solve in one kernel the registers cap residency at two 256-thread blocks
 // per SM and some values spill; the blocks of a cluster then wait at the
 // barriers of a pass whose tiles they do not share evenly, while the
