@@ -20,7 +20,7 @@
 //
 // Operator FP64, mixed-radix passes / these: 500 x 300 49.2 / 22.6 us, 1000^2
 // 63.6 / 50, 167^2 2750 / 33, 511 x 256 565 / 20.5.  Bound by the stages'
-// latency on small grids: radices up to 5, 6 or 9 only gave the same times up to
+// latency and instruction fetches on small grids: radices up to 5, 6 or 9 only gave the same times up to
 // 500^2 and lost at 1000^2 (47 -> 58-63).
 #pragma once
 #include "cm_fft_p2.cuh"
