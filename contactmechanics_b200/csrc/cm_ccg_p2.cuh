@@ -524,8 +524,10 @@ __global__ void __launch_bounds__(CM_EW_THREADS) k_ew_gsum(CcgArgs<R> a) {
 
 // Force update, projection onto [0, H] and the constraint bookkeeping
 // (ConstrainedConjugateGradients.py:296, 320-389)
+// (three blocks per SM: unbounded, the FP64 pass takes 122 registers and two,
+// and the grid, the order of its sums with it, follows the resident blocks)
 template <typename R, int U, bool P2>
-__global__ void __launch_bounds__(CM_EW_THREADS) k_ew_update(CcgArgs<R> a) {
+__global__ void __launch_bounds__(CM_EW_THREADS, 3) k_ew_update(CcgArgs<R> a) {
   typedef Vec16<R> VR;
   constexpr int V = VR::V;
   const EwIndex<P2> ix = ew_index<P2>(a);
