@@ -22,6 +22,7 @@ CM_ERR_BISECT = 7
 CM_ERR_BISECT_CONV = 8
 CM_ERR_TIMEOUT = 9
 CM_ERR_STOPPED = 10
+CM_ERR_GAVE_UP = 11
 
 CM_PERIODIC = 0
 CM_FREE = 1
@@ -123,6 +124,7 @@ SIGNATURES = {
     "cm_apply_periodic_noalloc": (_i, [_i, _i, ctypes.c_double, ctypes.c_double, ctypes.c_double,
                                        ctypes.c_double, _i, _vp, _vp, _vp]),
     "cm_selftest_grid_barrier": (_i, [_i, _i, ctypes.c_double, ctypes.POINTER(_i)]),
+    "cm_selftest_operator_barrier": (_i, [_vp, _i, _i, ctypes.c_double]),
     "cm_tuning_set_tiles": (_i, [_i, _i, _i]),
     "cm_tuning_set_batch_threads": (_i, [_i, _i]),
     "cm_tuning_get": (_i, [_i, _i, ctypes.POINTER(_i), ctypes.POINTER(_i)]),

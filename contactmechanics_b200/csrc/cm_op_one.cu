@@ -28,17 +28,26 @@ CM_DEVINL void one_release(GridBarrier* bar) {
   }
 }
 
-// A barrier gave up (a block was not scheduled for two seconds): the result
-// says so.
+// This block's wait gave up, or saw that another's had (a block was not
+// scheduled for two seconds): NaN in the rows that the block would have
+// written, tiles of `rows` of them, and the plan's word that the host reads
+// before the next call.  Blocks that got through the last barrier write their
+// own rows, whose inputs are complete; so every row is one or the other.
 template <typename R>
-__device__ __noinline__ void one_failed(const OpArgs<R>& a) {
-  for (int x = blockIdx.x; x < a.out_rows; x += gridDim.x)
-    for (int y = threadIdx.x; y < a.out_cols; y += T) a.out[(size_t)x * a.out_ld + y] = (R)NAN;
+__device__ __noinline__ void one_failed(const OpArgs<R>& a, int rows, int* gave_up) {
+  for (int xt = rows * blockIdx.x; xt < a.out_rows; xt += rows * gridDim.x)
+    for (int x = xt; x < min(xt + rows, a.out_rows); ++x)
+      for (int y = threadIdx.x; y < a.out_cols; y += T) a.out[(size_t)x * a.out_ld + y] = (R)NAN;
+  if (threadIdx.x == 0) {
+    *(volatile int*)gave_up = 1;
+    __threadfence_system();
+  }
 }
 
 template <typename R, int L>
 __global__ void __launch_bounds__(T, 1)
-k_op_one(const __grid_constant__ OpArgs<R> a, const __grid_constant__ SoloX X, int elems, GridBarrier* bar) {
+k_op_one(const __grid_constant__ OpArgs<R> a, const __grid_constant__ SoloX X, int elems, GridBarrier* bar,
+         long long limit, int* gave_up) {
   typedef typename CT<R>::C C;
   typedef SoloRow<L> Sh;
   typedef typename Sh::P P;
@@ -76,10 +85,10 @@ k_op_one(const __grid_constant__ OpArgs<R> a, const __grid_constant__ SoloX X, i
     }
     __syncthreads();
   }
-  bool alive = solo_barrier(bar, b, &ok);
+  bool alive = solo_barrier(bar, b, &ok, limit);
   if (alive) {
     solo_col_any<R>(X, fx, a, a.out_rows, twx, bufA, bufB);
-    alive = solo_barrier(bar, b, &ok);
+    alive = solo_barrier(bar, b, &ok, limit);
   }
   if (alive) {
 #pragma unroll 1
@@ -101,7 +110,7 @@ k_op_one(const __grid_constant__ OpArgs<R> a, const __grid_constant__ SoloX X, i
       __syncthreads();
     }
   } else {
-    one_failed(a);
+    one_failed(a, 2 * NP, gave_up);
   }
   one_release(bar);
 }
@@ -147,10 +156,10 @@ SoloPlan op_one_plan(int nx, int ny, int lx, int ly, const GenFft& gx) {
 
 template <typename R>
 int op_one_launch(const OpArgs<R>& a, int lx, int ly, const GenFft& gx, const SoloPlan& sp,
-                  GridBarrier* bar, cudaStream_t s) {
+                  GridBarrier* bar, long long limit, int* gave_up, cudaStream_t s) {
   const SoloX X = solo_x<R>(lx, gx);
   switch (ly) {
-#define CM_CASE(L) case L: return solo_cooperative(k_op_one<R, L>, sp, s, a, X, sp.elems, bar);
+#define CM_CASE(L) case L: return solo_cooperative(k_op_one<R, L>, sp, s, a, X, sp.elems, bar, limit, gave_up);
     CM_ONE_CASES(CM_CASE)
 #undef CM_CASE
     default: return -1;
@@ -160,6 +169,6 @@ int op_one_launch(const OpArgs<R>& a, int lx, int ly, const GenFft& gx, const So
 #define CM_INST(R)                                                                    \
   template SoloPlan op_one_plan<R>(int, int, int, int, const GenFft&);                \
   template int op_one_launch<R>(const OpArgs<R>&, int, int, const GenFft&, const SoloPlan&, \
-                                GridBarrier*, cudaStream_t);
+                                GridBarrier*, long long, int*, cudaStream_t);
 CM_INST(float)
 CM_INST(double)

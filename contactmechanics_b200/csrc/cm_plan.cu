@@ -561,6 +561,7 @@ struct Work {
   double* solo_partials = nullptr;
   SoloPlan one;             // launch shape of the one-launch operator (cm_op_one.cu)
   GridBarrier* one_bar = nullptr;
+  long long one_limit = CM_BARRIER_TIMEOUT_CYCLES;  // of its next launch's waits
   cudaGraphExec_t graph[2] = {nullptr, nullptr};  // [bisect passes]
   int graph_iters[2] = {0, 0};
   int graph_variant[2] = {0, 0};  // ccg_args.u_rows and fuse_gsum the graph was captured with
@@ -585,6 +586,7 @@ struct cm_plan {
   // pinned host states: [0] readback, [1] and [2] staging of the FP32 and FP64
   // initial states (a pageable source would make each copy wait for the stream)
   CcgState* h_state = nullptr;
+  int* gave_up = nullptr;  // behind them: set by an operator launch whose barrier gave up
   std::vector<void*> allocs;
   // stepping interface: phase of the solve this plan holds
   int phase = 0;          // 0 none, 1 FP32, 2 FP64
@@ -891,7 +893,8 @@ static int launch_plain(cm_plan* p, Work<R>& w, int mode, int table_sel, const R
       a.cg_only = 0;
       a.fwd_real = nullptr;
       if (w.one.grid && !per_pass) {
-        if (op_one_launch<R>(a, lx, ly, p->gx, w.one, w.one_bar, s) == 0) {
+        if (op_one_launch<R>(a, lx, ly, p->gx, w.one, w.one_bar, w.one_limit, p->gave_up, s) == 0) {
+          w.one_limit = CM_BARRIER_TIMEOUT_CYCLES;
           g_launches += 1;
           return CM_OK;
         }
@@ -951,6 +954,16 @@ static int forward_real_p2(cm_plan* p, const double* in, double* out, cudaStream
   const int rc = op_p2_fwd_real<double>(a, lx, ly, s);
   if (rc == 0) g_launches += 2;
   return rc > 0 ? CM_ERR_CUDA : rc;
+}
+
+// Reports, once, an operator launch of the plan whose barrier gave up (its
+// result holds NaN).  Only launches that have run are seen: a caller that does
+// not wait for its result learns of it with a later call.
+static int take_gave_up(cm_plan* p) {
+  volatile int* w = p->gave_up;
+  if (!*w) return CM_OK;
+  *w = 0;
+  return CM_ERR_GAVE_UP;
 }
 
 static int apply_dispatch(cm_plan* p, int op, int precision, const void* in, int in_rows, int in_cols,
@@ -1154,6 +1167,7 @@ template <typename R>
 static int ccg_init(cm_plan* p, Work<R>& w, const cm_ccg_params* prm, const SolveInput& in,
                     double rel_pentol, double rel_forcetol, int maxiter, cudaStream_t s) {
   set_smem_attrs<R>();
+  CKS(take_gave_up(p));
   CKS(ensure_ccg(p, w));
   CcgState st;
   initial_state(p, prm, rel_forcetol, maxiter, st);
@@ -1328,6 +1342,7 @@ static int run_ccg(cm_plan* p, Work<R>& w, const cm_ccg_params* prm, const Solve
     if (done_iters > maxiter + 2 * every) return CM_ERR_CUDA;  // state machine failed to stop
   }
   *fin = *p->h_state;
+  CKS(take_gave_up(p));  // of the solve's first displacement
   if (fin->status == CMS_TIMEOUT) return CM_ERR_TIMEOUT;
   if (fin->status == CMS_NAN) return CM_ERR_NAN;
   if (fin->status == CMS_BISECT_SIGN) return CM_ERR_BISECT;
@@ -1939,6 +1954,7 @@ const char* cm_status_string(int status) {
     case CM_ERR_BISECT: return "f(a) and f(b) must have different signs";
     case CM_ERR_BISECT_CONV: return "Failed to converge after 100 iterations";
     case CM_ERR_TIMEOUT: return "solve exceeded its time budget";
+    case CM_ERR_GAVE_UP: return "a wait of an earlier operator launch ran out: its result holds NaN";
     case CM_ERR_STOPPED: return "stopped by the per-iteration observer";
     default: return "unknown status";
   }
@@ -1988,10 +2004,12 @@ int cm_plan_create(const cm_plan_desc* desc, void* stream, cm_plan** out) {
       return fail(CM_ERR_CUDA);
     p->own_stream = true;
   }
-  if (cudaMallocHost(&p->h_state, 3 * sizeof(CcgState)) != cudaSuccess) {
+  if (cudaMallocHost(&p->h_state, 3 * sizeof(CcgState) + sizeof(int)) != cudaSuccess) {
     p->h_state = nullptr;
     return fail(CM_ERR_OOM);
   }
+  p->gave_up = reinterpret_cast<int*>(p->h_state + 3);
+  *p->gave_up = 0;
   if ((rc = init_work<double>(p, p->w64)) != CM_OK) return fail(rc);
   if ((rc = init_work<float>(p, p->w32)) != CM_OK) return fail(rc);
   // work items (0, i): every launch on this plan covers tiles 0..n-1 of slot 0
@@ -2118,6 +2136,7 @@ int cm_apply(cm_plan* p, int op, int precision, const void* in, int in_rows, int
   if (out_rows < 1 || out_rows > p->nx || out_cols < 1 || out_cols > p->ny || out_ld < out_cols)
     return CM_ERR_SHAPE;
   cudaStream_t s = stream ? (cudaStream_t)stream : p->stream;
+  CKS(take_gave_up(p));
   return apply_dispatch(p, op, precision, in, in_rows, in_cols, in_ld, out, out_rows, out_cols, out_ld, s);
 }
 
@@ -2720,6 +2739,22 @@ int cm_selftest_grid_barrier(int blocks, int phantom, double limit_us, int* gave
   cudaFree(d);
   *gave_up = h.gave_up;
   return rc;
+}
+
+int cm_selftest_operator_barrier(cm_plan* p, int precision, int missing, double limit_us) {
+  if (!p || (precision != CM_FP64 && precision != CM_FP32) || missing < 1 || missing > (1 << 20) ||
+      !(limit_us > 0) || limit_us > 1e7)
+    return CM_ERR_ARG;
+  GridBarrier* bar = precision == CM_FP64 ? p->w64.one_bar : p->w32.one_bar;
+  if (!bar) return CM_ERR_ARG;
+  int dev = 0, khz = 0;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&khz, cudaDevAttrClockRate, dev));
+  const unsigned count = 0u - (unsigned)missing;
+  CK(cudaDeviceSynchronize());  // no launch is at the barrier
+  CK(cudaMemcpy(&bar->count, &count, sizeof(count), cudaMemcpyHostToDevice));
+  (precision == CM_FP64 ? p->w64.one_limit : p->w32.one_limit) = (long long)(limit_us * 1e-3 * khz) + 1;
+  return CM_OK;
 }
 
 int cm_ccg_profile(cm_plan* p, const cm_ccg_params* prm, const double* h, int iters,

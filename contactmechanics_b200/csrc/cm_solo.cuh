@@ -112,7 +112,8 @@ CM_DEVINL void ld_acquire_pair(const GridBarrier* bar, unsigned& count, unsigned
 // Every block of the grid meets.  The first thread's arrival releases what
 // the block wrote before; its last poll acquires what the others wrote.  The
 // word after the count (GridBarrier::gen) carries the abort of this barrier.
-CM_DEVINL bool solo_barrier(GridBarrier* bar, SoloBarrier& b, int* ok_sm) {
+CM_DEVINL bool solo_barrier(GridBarrier* bar, SoloBarrier& b, int* ok_sm,
+                            long long limit = CM_BARRIER_TIMEOUT_CYCLES) {
   b.target += gridDim.x;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -124,7 +125,7 @@ CM_DEVINL bool solo_barrier(GridBarrier* bar, SoloBarrier& b, int* ok_sm) {
       ld_acquire_pair(bar, count, abort);
       if (abort) { ok = 0; break; }
       if ((int)(count - b.target) >= 0) break;
-      if (clock64() - t0 > CM_BARRIER_TIMEOUT_CYCLES) {
+      if (clock64() - t0 > limit) {
         atomicExch(&bar->gen, 1u);
         ok = 0;
         break;

@@ -44,6 +44,7 @@ extern "C" {
 #define CM_ERR_BISECT_CONV 8  /* offset bisection did not converge (RuntimeError) */
 #define CM_ERR_TIMEOUT 9      /* a solve exceeded its host-side time budget */
 #define CM_ERR_STOPPED 10     /* the per-iteration observer asked the solve to stop */
+#define CM_ERR_GAVE_UP 11     /* a wait of an earlier operator launch on the plan ran out (cm_apply) */
 
 /* substrate kinds */
 #define CM_PERIODIC 0
@@ -200,6 +201,12 @@ int cm_plan_greens_host(cm_plan* plan, double* out_host);
  * the Hockney zero padding; the output region [0,out_rows) x [0,out_cols) is
  * written with leading dimension out_ld.  precision selects float or double
  * buffers (CM_FP64 / CM_FP32).
+ *
+ * On small domains (sides 2^k of 64 to 1024, at most 2^18 points) the operator
+ * is one launch whose blocks wait for one another.  Should such a wait run out
+ * (about two seconds without all blocks running), the rows not computed hold
+ * NaN, and the next cm_apply or solve on the plan that starts once the launch
+ * has ended does nothing but report it, once, as CM_ERR_GAVE_UP.
  */
 int cm_apply(cm_plan* plan, int op, int precision, const void* in_dev, int in_rows,
              int in_cols, int in_ld, void* out_dev, int out_rows, int out_cols, int out_ld,
@@ -348,6 +355,15 @@ int cm_apply_periodic_noalloc(int nx, int ny, double sx, double sy, double young
  * counterpart.
  */
 int cm_selftest_grid_barrier(int blocks, int phantom, double limit_us, int* gave_up);
+
+/*
+ * Makes the next one-launch cm_apply of `plan` in `precision` wait for
+ * `missing` arrivals that never come, for at most `limit_us` microseconds of
+ * SM clock: tests see the error of cm_apply above, and that the call after it
+ * works.  CM_ERR_ARG when the plan's operator is not one launch.
+ * Instrumentation; no reference counterpart.
+ */
+int cm_selftest_operator_barrier(cm_plan* plan, int precision, int missing, double limit_us);
 
 /*
  * Tuning of the per-pass kernels that batched solves (cm_ccg_solve_batch),
