@@ -430,6 +430,10 @@ struct alignas(16) Vec16 {
 };
 
 #define CM_EW_THREADS 256
+// Blocks per SM of the element-wise passes, guaranteed by their launch bounds
+// and no more: the grid is the order of their sums, which the plastic mask of
+// a solve with a hardness shows.
+#define CM_EW_BLOCKS 3
 
 // vector j of the topography: element index (topography) and displacement
 // index.  P2: the vectors per topography row are a power of two (a shift
@@ -470,7 +474,7 @@ inline bool ew_pow2(const CcgArgs<R>& a) { return (a.ew_vpr.d & (a.ew_vpr.d - 1)
 
 // G = sum over the CG area of g^2 (ConstrainedConjugateGradients.py:273-279)
 template <typename R, int U, bool P2>
-__global__ void __launch_bounds__(CM_EW_THREADS) k_ew_gsum(CcgArgs<R> a) {
+__global__ void __launch_bounds__(CM_EW_THREADS, CM_EW_BLOCKS) k_ew_gsum(CcgArgs<R> a) {
   typedef Vec16<R> VR;
   constexpr int V = VR::V;
   const EwIndex<P2> ix = ew_index<P2>(a);
@@ -524,10 +528,9 @@ __global__ void __launch_bounds__(CM_EW_THREADS) k_ew_gsum(CcgArgs<R> a) {
 
 // Force update, projection onto [0, H] and the constraint bookkeeping
 // (ConstrainedConjugateGradients.py:296, 320-389)
-// (three blocks per SM: unbounded, the FP64 pass takes 122 registers and two,
-// and the grid, the order of its sums with it, follows the resident blocks)
+// (unbounded, the FP64 pass takes 122 registers and two blocks per SM)
 template <typename R, int U, bool P2>
-__global__ void __launch_bounds__(CM_EW_THREADS, 3) k_ew_update(CcgArgs<R> a) {
+__global__ void __launch_bounds__(CM_EW_THREADS, CM_EW_BLOCKS) k_ew_update(CcgArgs<R> a) {
   typedef Vec16<R> VR;
   constexpr int V = VR::V;
   const EwIndex<P2> ix = ew_index<P2>(a);

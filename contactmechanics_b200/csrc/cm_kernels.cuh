@@ -884,10 +884,18 @@ CM_DEVINL void begin_tile(const Slot<R>* __restrict__ Sp, int tile, const R* __r
   });
 }
 
+// Blocks per SM of the begin pass of a single solve, guaranteed by its launch
+// bounds.  A constant, because the grid is the order of its sums: a solve with
+// a hardness started from given forces shows it in its last bits (a register
+// more had made it three blocks in FP64, and with them 2048 x 512 another sum;
+// the pass of 1500^2 26.2 -> 30.5 us, 27.2 bounded).
+template <typename R>
+constexpr int begin_blocks() { return sizeof(R) == 8 ? 4 : 3; }
+
 // Start of an iteration: contact areas, raw-gap sums, step kind and offset
 // (ConstrainedConjugateGradients.py:239-270, 300-318).
 template <typename R>
-__global__ void __launch_bounds__(CM_THREADS)
+__global__ void __launch_bounds__(CM_THREADS, begin_blocks<R>())
 k_ccg_begin(const Slot<R>* __restrict__ slots, const int2* __restrict__ items, int strided) {
   const int2 item = items[strided > 0 ? 0 : blockIdx.x];
   const Slot<R>* __restrict__ Sp = slots + item.x;

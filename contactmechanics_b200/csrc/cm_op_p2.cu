@@ -303,7 +303,7 @@ int ccg_p2_ew_blocks_per_sm(const CcgArgs<R>& a) {
                           : (const void*)k_ew_gsum<R, CM_EW_UNROLL, false>,
                        p2 ? (const void*)k_ew_update<R, CM_EW_UNROLL, true>
                           : (const void*)k_ew_update<R, CM_EW_UNROLL, false>};
-  int n = 1 << 30;
+  int n = CM_EW_BLOCKS;  // (at most, for the order of the sums)
   for (const void* k : ks) {
     int b = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, CM_EW_THREADS, 0) != cudaSuccess) return -1;

@@ -827,6 +827,7 @@ static int ensure_ccg(cm_plan* p, Work<R>& w) {
       for (int k = 0; k < 4; ++k) {
         int per_sm = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ks[k], CM_THREADS, 0));
+        if (k == 0) per_sm = std::min(per_sm, begin_blocks<R>());
         w.ew_grid[k] = std::max(1, std::min(w.nt_comp, per_sm * nsm));
       }
       // all bisection passes of an iteration in one cooperative launch
