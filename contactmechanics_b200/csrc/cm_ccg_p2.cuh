@@ -23,6 +23,23 @@
 #pragma once
 #include "cm_op_p2.cuh"
 
+// The end of the forward row pass of the forces: their sum and largest value,
+// and the scalar step.  Out of line on rows of 2^k points, where its registers
+// make the pass spill (FP32 rows of 4096: 88 bytes, 4096^2 116.7 us, 94.4 so;
+// FP64 175 -> 168); inlined on rows of 3 * 2^m, which have room (FP64 6144^2
+// 428 us, 436 out of line).
+static CM_DEVINL void force_finish_inline(CcgState* st, double* partials, unsigned int* counter,
+                                          double s_f, double fmax_in) {
+  double v[2] = {s_f, fmax_in};
+  const int kinds[2] = {RED_SUM, RED_MAX};
+  tile_finish<2>(st, partials, counter, blockIdx.x, gridDim.x, v, kinds,
+                 [&](CcgState& s, double (&r)[2]) { fin_force(s, r); });
+}
+static __device__ __noinline__ void force_finish(CcgState* st, double* partials,
+                                                 unsigned int* counter, double s_f, double fmax_in) {
+  force_finish_inline(st, partials, counter, s_f, fmax_in);
+}
+
 template <typename R, int MODE, int LOGN>
 __global__ void __launch_bounds__(OpShape<R, LOGN>::THREADS, OpShape<R, LOGN>::MINB)
 k_ccg_row_fwd(CcgArgs<R> a) {
@@ -203,11 +220,10 @@ k_ccg_row_fwd(CcgArgs<R> a) {
     const int kinds[1] = {RED_SUM};
     tile_finish<1>(st, a.partials, a.counter, blockIdx.x, gridDim.x, vr, kinds,
                    [&](CcgState& s, double (&r)[1]) { s.sum_cgt = r[0]; });
+  } else if constexpr (P::F == 1) {
+    force_finish(st, a.partials, a.counter, acc, (double)amax);
   } else {
-    double vr[2] = {acc, (double)amax};
-    const int kinds[2] = {RED_SUM, RED_MAX};
-    tile_finish<2>(st, a.partials, a.counter, blockIdx.x, gridDim.x, vr, kinds,
-                   [&](CcgState& s, double (&r)[2]) { fin_force(s, r); });
+    force_finish_inline(st, a.partials, a.counter, acc, (double)amax);
   }
 }
 
@@ -526,6 +542,18 @@ __global__ void __launch_bounds__(CM_EW_THREADS, CM_EW_BLOCKS) k_ew_gsum(CcgArgs
                  [&](CcgState& s, double (&r)[1]) { fin_gsum(s, r); });
 }
 
+// The end of the force update: the sums and the scalar step.  Out of line:
+// inlined, its registers make the pass spill 40 bytes in FP64 (2048^2 40.9 us,
+// 35.7 so; 8192^2 436 -> 389).
+static __device__ __noinline__ void update_finish(CcgState* st, double* partials,
+                                                  unsigned int* counter, double n_fl, double min_fn,
+                                                  double max_t, double s_fp, double n_nc) {
+  double v[5] = {n_fl, min_fn, max_t, s_fp, n_nc};
+  const int kinds[5] = {RED_SUM, RED_MIN, RED_MAX, RED_SUM, RED_SUM};
+  tile_finish<5>(st, partials, counter, blockIdx.x, gridDim.x, v, kinds,
+                 [&](CcgState& s, double (&r)[5]) { fin_update(s, r); });
+}
+
 // Force update, projection onto [0, H] and the constraint bookkeeping
 // (ConstrainedConjugateGradients.py:296, 320-389)
 // (unbounded, the FP64 pass takes 122 registers and two blocks per SM)
@@ -537,14 +565,12 @@ __global__ void __launch_bounds__(CM_EW_THREADS, CM_EW_BLOCKS) k_ew_update(CcgAr
   const long nvec = (long)a.tx * a.ty / V;
   pdl_wait();
   CcgState* st = a.st;
-  CcgView cv;
-  load_view(st, cv);
+  if (st->done) return;
+  const int par = st->parity & 1, has_h = st->p.has_h, branch = st->branch;
+  const double H = st->p.H;
+  const R off = (R)st->offset;
+  const R tau = (R)st->tau;
   const double mix = st->cur_mixfac;
-  if (cv.done) return;
-  const int par = cv.par & 1, has_h = cv.has_h, branch = cv.branch;
-  const double H = cv.H;
-  const R off = (R)cv.offset;
-  const R tau = (R)cv.tau;
   const R* __restrict__ f = a.f[par];
   R* __restrict__ fo = a.f[par ^ 1];
   const R* __restrict__ t = a.t;
@@ -611,8 +637,6 @@ __global__ void __launch_bounds__(CM_EW_THREADS, CM_EW_BLOCKS) k_ew_update(CcgAr
     }
   }
   pdl_trigger();
-  double v[5] = {(double)a_fl, (double)min_fn + H, (double)max_t, s_fp, (double)n_nc};
-  const int kinds[5] = {RED_SUM, RED_MIN, RED_MAX, RED_SUM, RED_SUM};
-  tile_finish<5>(st, a.partials, a.counter, blockIdx.x, gridDim.x, v, kinds,
-                 [&](CcgState& s, double (&r)[5]) { fin_update(s, r); });
+  update_finish(st, a.partials, a.counter, (double)a_fl, (double)min_fn + H, (double)max_t, s_fp,
+                (double)n_nc);
 }
