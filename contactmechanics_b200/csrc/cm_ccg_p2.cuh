@@ -325,67 +325,77 @@ k_ccg_row_inv(CcgArgs<R> a) {
       for (int w = 0; w < 2; ++w) {
         const int x = xa + w;
         if (x >= rows_total) continue;
-        // every input of the row's E elements first, from addresses that are
-        // valid without a test (a branch around each load, or a use of one
-        // inside it, makes the row's loads wait for one another: 8700 cycles a
-        // tile of 16 x 256 in FP64 instead of 2500), then the stores
+        // every input of a chunk of the row's elements first, from addresses
+        // that are valid without a test (a branch around each load, or a use of
+        // one inside it, makes the row's loads wait for one another: 8700
+        // cycles a tile of 16 x 256 in FP64 instead of 2500), then the stores.
+        // The whole row at once, but for more than 8 elements in the 128
+        // registers of 512 resident threads, where FP64 (1268 bytes of spills
+        // at 8192; 8192^2 1536 us whole, 861 in fours, 6144^2 762 and 618, free
+        // 4096^2 955 and 645) and FP32 rows of 8192 (472 and 411 in eights)
+        // spill; 12 FP32 elements fit (6144^2 232 us, 262 in fours).
+        constexpr int CH = Sh::E <= 8 || Sh::THREADS * Sh::MINB < 512 ? Sh::E
+                           : sizeof(R) == 8 ? 4 : Sh::E % 8 == 0 ? 8 : Sh::E;
         const bool in_x = x < tx;
-        R uo[Sh::E], hv[Sh::E], fn[Sh::E], fa[Sh::E];
 #pragma unroll
-        for (int q = 0; q < Sh::E; ++q) uo[q] = u_io[(size_t)x * N + tt + q * P::TPS];
-        if (in_x) {
-          const size_t rb = (size_t)x * ty;
+        for (int q0 = 0; q0 < Sh::E; q0 += CH) {
+          R uo[CH], hv[CH], fn[CH], fa[CH];
 #pragma unroll
-          for (int q = 0; q < Sh::E; ++q) {
-            const int y = tt + q * P::TPS;
-            const size_t ic = rb + (y < ty ? y : 0);
-            hv[q] = h_in[ic];
-            fn[q] = fn_buf[ic];
-          }
-          // the force at the iteration's start, or the mixing step's mask
-          if (cv.branch == 0) {
+          for (int q = 0; q < CH; ++q) uo[q] = u_io[(size_t)x * N + tt + (q0 + q) * P::TPS];
+          if (in_x) {
+            const size_t rb = (size_t)x * ty;
 #pragma unroll
-            for (int q = 0; q < Sh::E; ++q) {
-              const int y = tt + q * P::TPS;
-              fa[q] = fa_buf[rb + (y < ty ? y : 0)];
+            for (int q = 0; q < CH; ++q) {
+              const int y = tt + (q0 + q) * P::TPS;
+              const size_t ic = rb + (y < ty ? y : 0);
+              hv[q] = h_in[ic];
+              fn[q] = fn_buf[ic];
             }
-          } else {
+            // the force at the iteration's start, or the mixing step's mask
+            if (cv.branch == 0) {
 #pragma unroll
-            for (int q = 0; q < Sh::E; ++q) {
-              const int y = tt + q * P::TPS;
-              fa[q] = (R)gneg[rb + (y < ty ? y : 0)];
-            }
-          }
-        }
+              for (int q = 0; q < CH; ++q) {
+                const int y = tt + (q0 + q) * P::TPS;
+                fa[q] = fa_buf[rb + (y < ty ? y : 0)];
+              }
+            } else {
 #pragma unroll
-        for (int q = 0; q < Sh::E; ++q) {
-          const int y = tt + q * P::TPS;
-          const R val = w ? v[q].y : v[q].x;
-          du = fmax(du, fabs(val - uo[q]));
-          u_io[(size_t)x * N + y] = val;
-          if (in_x && y < ty) {
-            const bool cc = cv.branch == 0 ? (fa[q] < 0) && (!cv.has_h || fa[q] > hdn) : fa[q] != 0;
-            const R pen = (hv[q] + off) - val;
-            pmax = fmax(pmax, cc ? pen : (R)0);
-            const bool c0 = fn[q] < 0;
-            const bool c = c0 && (!cv.has_h || fn[q] > hdn);
-            const R g = val - hv[q];
-            n_c += c0;
-            n_cg += c;
-            if (c) s_cg += (double)g;
-            if (a.fuse_gsum) {
-              // the reference sums c g^2 over the whole topography, so a NaN
-              // gap outside the contact set makes G NaN as well
-              const double gs = (double)g - cv.offset;
-              if (c) {
-                s1 += gs;
-                s2 += gs * gs;
-              } else if (isnan(g)) {
-                s2 += (double)g;
+              for (int q = 0; q < CH; ++q) {
+                const int y = tt + (q0 + q) * P::TPS;
+                fa[q] = (R)gneg[rb + (y < ty ? y : 0)];
               }
             }
-            gmax = fmax(gmax, g);
-            gmin = fmin(gmin, g);
+          }
+#pragma unroll
+          for (int q = 0; q < CH; ++q) {
+            const int y = tt + (q0 + q) * P::TPS;
+            const R val = w ? v[q0 + q].y : v[q0 + q].x;
+            du = fmax(du, fabs(val - uo[q]));
+            u_io[(size_t)x * N + y] = val;
+            if (in_x && y < ty) {
+              const bool cc = cv.branch == 0 ? (fa[q] < 0) && (!cv.has_h || fa[q] > hdn) : fa[q] != 0;
+              const R pen = (hv[q] + off) - val;
+              pmax = fmax(pmax, cc ? pen : (R)0);
+              const bool c0 = fn[q] < 0;
+              const bool c = c0 && (!cv.has_h || fn[q] > hdn);
+              const R g = val - hv[q];
+              n_c += c0;
+              n_cg += c;
+              if (c) s_cg += (double)g;
+              if (a.fuse_gsum) {
+                // the reference sums c g^2 over the whole topography, so a NaN
+                // gap outside the contact set makes G NaN as well
+                const double gs = (double)g - cv.offset;
+                if (c) {
+                  s1 += gs;
+                  s2 += gs * gs;
+                } else if (isnan(g)) {
+                  s2 += (double)g;
+                }
+              }
+              gmax = fmax(gmax, g);
+              gmin = fmin(gmin, g);
+            }
           }
         }
       }
