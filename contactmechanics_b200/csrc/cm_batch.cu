@@ -191,7 +191,7 @@ CM_DEVINL void batch_plain_op(BatchShared& sh, unsigned rank, unsigned char* sme
     stage_fft(sh.fd, S.fy, tws, S.twy, S.ny);
     for_tiles((out_rows + S.row_tile - 1) / S.row_tile, rank, [&](int tile) {
       NextIter no_next;
-      row_inv_tile<R, MODE_PLAIN>(&S, cv, tile, sh.fd, tws, buf, scratch, d0, d1, no_next, false);
+      row_inv_tile<R, MODE_PLAIN, false>(&S, cv, tile, sh.fd, tws, buf, scratch, d0, d1, no_next, false);
     });
   }
   cluster_sync();
@@ -287,7 +287,7 @@ CM_DEVINL void batch_phase(BatchShared& sh, int& rb, unsigned rank, unsigned cha
       stage_fft(sh.fd, S.fy, tws, S.twy, S.ny);
       for_tiles(S.nt_rowt, rank, [&](int tile) {
         NextIter no_next;
-        row_inv_tile<R, MODE_T>(&S, cv, tile, sh.fd, tws, rbuf, rscr, s_rt, u1, no_next, false);
+        row_inv_tile<R, MODE_T, false>(&S, cv, tile, sh.fd, tws, rbuf, rscr, s_rt, u1, no_next, false);
       });
       double v[2] = {s_gt, s_rt};
       const int kinds[2] = {RED_SUM, RED_SUM};
@@ -331,7 +331,7 @@ CM_DEVINL void batch_phase(BatchShared& sh, int& rb, unsigned rank, unsigned cha
       stage_fft(sh.fd, S.fy, tws, S.twy, S.ny);
       for_tiles(S.nt_rowd, rank, [&](int tile) {
         NextIter no_next;
-        row_inv_tile<R, MODE_F>(&S, cv, tile, sh.fd, tws, rbuf, rscr, du, pen, no_next, false);
+        row_inv_tile<R, MODE_F, false>(&S, cv, tile, sh.fd, tws, rbuf, rscr, du, pen, no_next, false);
       });
       double v[4] = {s_f, m_f, du, pen};
       const int kinds[4] = {RED_SUM, RED_MAX, RED_MAX, RED_MAX};

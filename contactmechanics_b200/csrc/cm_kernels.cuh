@@ -465,11 +465,20 @@ CM_DEVINL void row_fwd_tile(const Slot<R>* __restrict__ Sp, const CcgView& cv, i
   }
 }
 
-// Registers of the FP64 transform passes: three 256-thread blocks per SM (the
-// 64-solve batch's row passes 70 -> 66, 62 -> 57, 56 -> 49 us, columns 45 -> 39),
-// but for the displacement pass, whose epilogue spills there (121 -> 129).
-template <typename R, int MODE, bool INV>
-constexpr int pass_regs() { return sizeof(R) == 8 && !(INV && MODE == MODE_F) ? 80 : 128; }
+// Registers of the transform passes: three 256-thread blocks per SM, six of
+// 128.  FP64 spills there (150-400 bytes a thread) and is faster all the same
+// in a batch (64 solves: row passes 70 -> 66, 62 -> 57, 56 -> 49 us, columns 45
+// -> 39), no slower in a single solve, whose shared memory leaves two blocks
+// (1500^2: rows 62.9 and 62.5, columns 61.2 and 57.7 us).  FP32 takes 104 to
+// 119 unbounded and spills nothing at 80 (1200^2 forward, column, inverse pass
+// 38.8, 34.6, 38.0 us unbounded, 28.5, 27.3, 28.7 so; batches alike).  The
+// displacement pass, whose epilogue holds more, is unbounded in FP64 (64 solves
+// 121 us, 129 at 80) and in batches; in single FP32 solves it takes 96 (1200^2
+// 45.6 -> 34.8 us).
+template <typename R, int MODE, bool INV, bool FUSABLE = false>
+constexpr int pass_regs() {
+  return !(INV && MODE == MODE_F) ? 80 : sizeof(R) == 8 || FUSABLE ? 128 : 96;
+}
 
 template <typename R, int MODE>
 __global__ void __maxnreg__((pass_regs<R, MODE, false>()))
@@ -632,13 +641,15 @@ CM_DEVINL void ccg_converge(CcgState& s, double maxdu_in, double maxpen_in) {
 // caller's buffer, or the CCG epilogue.  fd / tws / buf / scratch as for
 // row_fwd_tile.  a0 / a1 collect this thread's share of the tile's sums
 // (MODE_T: sum r t; MODE_F: max |du|, max penetration over the CG set).  fuse
-// (MODE_F): nx_it collects the next iteration's start of an elastic solve, from
-// the new displacement and the iteration's final force.
+// (MODE_F, FUSABLE): nx_it collects the next iteration's start of an elastic
+// solve, from the new displacement and the iteration's final force.  Launches
+// of which no solve does that take FUSABLE = false, which keeps two elements
+// in flight in FP64 (1500^2 73 us a launch, 108 with one).
 struct NextIter {
   int n_c = 0;                     // contact points
   double s_cg = 0, s1 = 0, s2 = 0; // sums over them of g, g - off, (g - off)^2
 };
-template <typename R, int MODE>
+template <typename R, int MODE, bool FUSABLE>
 CM_DEVINL void row_inv_tile(const Slot<R>* __restrict__ Sp, const CcgView& cv, int tile,
                             const FftDesc& fd, const typename CT<R>::C* tws,
                             typename CT<R>::C* buf, typename CT<R>::C* scratch, double& a0,
@@ -706,7 +717,7 @@ CM_DEVINL void row_inv_tile(const Slot<R>* __restrict__ Sp, const CcgView& cv, i
     const R off = (R)cv.offset;
     struct UF { R uo[2], fa[2], h[2], fn[2]; unsigned char gn[2]; };
     const bool topo = x0 < tx;  // else a tile of padding rows
-    batched_loop<sizeof(R) == 8 ? 1 : 2>(npairs * ny, [&](int e) {
+    batched_loop<FUSABLE && sizeof(R) == 8 ? 1 : 2>(npairs * ny, [&](int e) {
       const int p = fdiv(dny, e), y = e - p * ny, yy = y < ty ? y : 0;
       UF v;
 #pragma unroll
@@ -719,7 +730,7 @@ CM_DEVINL void row_inv_tile(const Slot<R>* __restrict__ Sp, const CcgView& cv, i
           v.h[w] = ldf(h + ic);
           if (cv.branch == 0) v.fa[w] = ldf(fa_buf + ic);
           else v.gn[w] = ldf(gneg + ic);
-          if (fuse) v.fn[w] = ldf(fn_buf + ic);
+          if (FUSABLE && fuse) v.fn[w] = ldf(fn_buf + ic);
         }
       }
       return v;
@@ -739,7 +750,7 @@ CM_DEVINL void row_inv_tile(const Slot<R>* __restrict__ Sp, const CcgView& cv, i
           else c = v.gn[w] != 0;
           const R pen = (v.h[w] + off) - val;
           a1 = fmax(a1, c ? (double)pen : 0.0);
-          if (fuse) {
+          if (FUSABLE && fuse) {
             const R g = val - v.h[w];
             // the reference sums c g^2 over the whole topography, so a NaN gap
             // outside the contact set makes G NaN as well
@@ -759,8 +770,8 @@ CM_DEVINL void row_inv_tile(const Slot<R>* __restrict__ Sp, const CcgView& cv, i
   }
 }
 
-template <typename R, int MODE>
-__global__ void __maxnreg__((pass_regs<R, MODE, true>()))
+template <typename R, int MODE, bool FUSABLE = false>
+__global__ void __maxnreg__((pass_regs<R, MODE, true, FUSABLE>()))
 k_row_inv(const Slot<R>* __restrict__ slots, const int2* __restrict__ items) {
   typedef typename CT<R>::C C;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -780,14 +791,14 @@ k_row_inv(const Slot<R>* __restrict__ slots, const int2* __restrict__ items) {
   stage_fft(fd, Sp->fy, tws, Sp->twy, ny);
   double a0 = 0.0, a1 = -INFINITY;  // MODE_T: sum r t ; MODE_F: max|du|, max penetration
   NextIter next;
-  const bool fuse = MODE == MODE_F && Sp->fuse;
-  row_inv_tile<R, MODE>(Sp, cv, item.y, fd, tws, buf, scratch, a0, a1, next, fuse);
+  const bool fuse = FUSABLE && Sp->fuse;
+  row_inv_tile<R, MODE, FUSABLE>(Sp, cv, item.y, fd, tws, buf, scratch, a0, a1, next, fuse);
   if (MODE == MODE_T) {
     double v[1] = {a0};
     const int kinds[1] = {RED_SUM};
     tile_finish<1>(st, Sp->partials, Sp->counter, item.y, Sp->nt_rowt, v, kinds,
                    [&](CcgState& s, double (&a)[1]) { fin_tau(s, a); });
-  } else if (MODE == MODE_F && fuse) {
+  } else if (FUSABLE && fuse) {
     double v[6] = {a0, a1, (double)next.n_c, next.s_cg, next.s1, next.s2};
     const int kinds[6] = {RED_MAX, RED_MAX, RED_SUM, RED_SUM, RED_SUM, RED_SUM};
     const double off64 = cv.offset;

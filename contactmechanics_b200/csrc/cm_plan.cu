@@ -664,6 +664,7 @@ static void set_smem_attrs_once() {
   cudaFuncSetAttribute(k_col<R, MODE_F>, cudaFuncAttributePreferredSharedMemoryCarveout, carve);
   cudaFuncSetAttribute(k_row_inv<R, MODE_T>, cudaFuncAttributePreferredSharedMemoryCarveout, carve);
   cudaFuncSetAttribute(k_row_inv<R, MODE_F>, cudaFuncAttributePreferredSharedMemoryCarveout, carve);
+  cudaFuncSetAttribute(k_row_inv<R, MODE_F, true>, cudaFuncAttributePreferredSharedMemoryCarveout, carve);
   cudaFuncSetAttribute(k_row_fwd<R, MODE_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
   cudaFuncSetAttribute(k_row_fwd<R, MODE_FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
   cudaFuncSetAttribute(k_row_fwd<R, MODE_T>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
@@ -675,6 +676,7 @@ static void set_smem_attrs_once() {
   cudaFuncSetAttribute(k_row_inv<R, MODE_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
   cudaFuncSetAttribute(k_row_inv<R, MODE_T>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
   cudaFuncSetAttribute(k_row_inv<R, MODE_F>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
+  cudaFuncSetAttribute(k_row_inv<R, MODE_F, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
 }
 
 template <typename R>
@@ -1427,6 +1429,7 @@ struct BatchDev {
   int* running = nullptr;  // count of running solves, then one done flag per solve
   size_t smem_row = 0, smem_col = 0;
   bool fuse = false;  // Slot::fuse of every slot
+  bool fuse_any = false;  // ... of some slot
   std::vector<void*> allocs;
   ~BatchDev() {
     for (void* a : allocs) cudaFree(a);
@@ -1504,7 +1507,8 @@ static void launch_iteration_batch(const BatchDev<R>& b, bool bisect, cudaStream
   k_ccg_update<R><<<b.n_items[0], CM_THREADS, 0, s>>>(S, b.items[0], 0);
   k_row_fwd<R, MODE_F><<<b.n_items[1], TT, b.smem_row, s>>>(S, b.items[1]);
   k_col<R, MODE_F><<<b.n_items[3], TT, b.smem_col, s>>>(S, b.items[3]);
-  k_row_inv<R, MODE_F><<<b.n_items[2], TT, b.smem_row, s>>>(S, b.items[2]);
+  if (b.fuse_any) k_row_inv<R, MODE_F, true><<<b.n_items[2], TT, b.smem_row, s>>>(S, b.items[2]);
+  else k_row_inv<R, MODE_F><<<b.n_items[2], TT, b.smem_row, s>>>(S, b.items[2]);
 }
 
 // Count the solves of a batch that have not finished; done flags after it.
@@ -1605,7 +1609,10 @@ static int lockstep_phase(int n, cm_plan* const* plans, const cm_ccg_params* par
   for (int i = 0; i < n; ++i) CKS(ensure_ccg(plans[i], work_of<R>(plans[i])));
   BatchDev<R> b;
   b.fuse = true;
-  for (int i = 0; i < n; ++i) b.fuse = b.fuse && !params[i].has_hardness;
+  for (int i = 0; i < n; ++i) {
+    b.fuse = b.fuse && !params[i].has_hardness;
+    b.fuse_any = b.fuse_any || !params[i].has_hardness;
+  }
   CKS(batch_build<R>(n, plans, b, s, [&](int i, Slot<R>& sl) {
     cm_plan* p = plans[i];
     sl.fuse = !params[i].has_hardness;
