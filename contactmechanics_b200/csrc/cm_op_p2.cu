@@ -83,13 +83,20 @@ int row_fwd(const OpArgs<R>& a, cudaStream_t s, bool launch = true) {
   }
 }
 
-template <typename R, int LOGX, int BASE>
+// blocks of shape Sh with a column group for each of their places
+template <typename Sh, typename R>
+int col_blocks(const OpArgs<R>& a) {
+  const int groups = (a.ny / 2 + Sh::W) / Sh::W;
+  return (groups + Sh::NG - 1) / Sh::NG;
+}
+
+template <typename R, int LOGX, int BASE, bool FEW>
 int prepare_col(KernelInfo& info) {
-  typedef ColShape<R, LOGX, BASE> Sh;
+  typedef ColShape<R, LOGX, BASE, FEW> Sh;
   if (info.ready) return info.grid_per_sm > 0 ? 0 : -1;
   const size_t smem = Sh::smem();
   if (smem > CM_SMEM_DYN_MAX) return -1;
-  const void* kernel = (const void*)k_op_col<R, LOGX, BASE>;
+  const void* kernel = (const void*)k_op_col<R, LOGX, BASE, FEW>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return 1;
   int per_sm = 0;
@@ -100,38 +107,44 @@ int prepare_col(KernelInfo& info) {
   return per_sm > 0 ? 0 : -1;
 }
 
-template <typename R, int LOGX, int BASE>
-int col_base(const OpArgs<R>& a, int groups, cudaStream_t s, bool launch) {
-  typedef ColShape<R, LOGX, BASE> Sh;
+template <typename R, int LOGX, int BASE, bool FEW = false>
+int col_base(const OpArgs<R>& a, cudaStream_t s, bool launch) {
+  typedef ColShape<R, LOGX, BASE, FEW> Sh;
   static KernelInfo info;
   int rc;
   {
     std::lock_guard<std::mutex> g(g_op_mu);
-    rc = prepare_col<R, LOGX, BASE>(info);
+    rc = prepare_col<R, LOGX, BASE, FEW>(info);
   }
   if (rc || !launch) return rc;
-  const int blocks = (groups + Sh::NG - 1) / Sh::NG;
+  const int blocks = col_blocks<Sh>(a);
   const int grid = std::max(1, std::min(blocks, info.grid_per_sm * sm_count()));
-  launch_pdl(k_op_col<R, LOGX, BASE>, grid, Sh::THREADS, Sh::smem(), s, a);
+  launch_pdl(k_op_col<R, LOGX, BASE, FEW>, grid, Sh::THREADS, Sh::smem(), s, a);
   return 0;
 }
 
 // column pass on the pair-major spectrum (k_op_col); LOGX: length code of the
 // columns (domain rows).  Short columns of a small grid, and of sides 3 * 2^m,
-// take small blocks (CM_COL_BASE_SHORT).
+// take small blocks (CM_COL_BASE_SHORT), long ones of few columns the shape for
+// them (ColShape).
 template <typename R, int LOGX>
 int col(const OpArgs<R>& a, cudaStream_t s, bool launch = true) {
   if constexpr (!len_fits<R, LOGX>()) {
     return -1;
   } else {
     typedef ColShape<R, LOGX> Sh;
-    const int units = a.ny / 2 + 1;
-    const int groups = (units + Sh::W - 1) / Sh::W;
+    typedef ColShape<R, LOGX, CM_COL_BASE, true> Few;
     if constexpr (Sh::NG > 1) {
-      if (LOGX >= 32 || 2 * ((groups + Sh::NG - 1) / Sh::NG) <= sm_count())
-        return col_base<R, LOGX, CM_COL_BASE_SHORT>(a, groups, s, launch);
+      if (LOGX >= 32 || 2 * col_blocks<Sh>(a) <= sm_count())
+        return col_base<R, LOGX, CM_COL_BASE_SHORT>(a, s, launch);
     }
-    return col_base<R, LOGX, CM_COL_BASE>(a, groups, s, launch);
+    if constexpr (Sh::NG == 1 && (Few::W != Sh::W || Few::TWO != Sh::TWO)) {
+      const int nsm = sm_count(), few = (col_blocks<Few>(a) + nsm - 1) / nsm,
+                waves = (col_blocks<Sh>(a) + Sh::MINB * nsm - 1) / (Sh::MINB * nsm);
+      if (5 * few <= (LOGX >= 32 ? 8 : 5) * waves)
+        return col_base<R, LOGX, CM_COL_BASE, true>(a, s, launch);
+    }
+    return col_base<R, LOGX, CM_COL_BASE>(a, s, launch);
   }
 }
 

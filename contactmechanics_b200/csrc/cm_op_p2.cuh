@@ -179,8 +179,14 @@ struct OpShape {
 
 // Column pass for columns of length code LOGX: 16 elements per thread for
 // 2^LOGX (3 x 2^LR for 3 * 2^m), groups of W = 2^LW columns with the column
-// index fastest across threads.
-template <typename R, int LOGX, int BASE = CM_COL_BASE>
+// index fastest across threads.  FEW: for grids of few columns, where two
+// buffers (one barrier an exchange) and, for them, a column less per group beat
+// whole sectors and pairs of blocks: as long as it takes no more waves of
+// blocks, or for 3 * 2^m no more than 8/5 times as many (FP64 operator 2048 x
+// 384 37.1 us, 29.6 so; 4096 x 256 33.0 and 26.1, 4096 x 384, two waves against
+// one, 50.4 and 57.9; 3072 x 256 31.3 and 23.2, 3072 x 768, three against two,
+// 70.3 and 64.6, 3072 x 1024, four against two, 70.7 and 76.3).
+template <typename R, int LOGX, int BASE = CM_COL_BASE, bool FEW = false>
 struct ColShape {
   typedef typename CT<R>::C C;
   static constexpr int LR = LenCode<LOGX>::F == 3 ? (sizeof(R) == 8 ? CM_T3_LR_F64 : CM_T3_LR_F32)
@@ -197,7 +203,7 @@ struct ColShape {
   // fewer if not even one buffer of them fits
   static constexpr int LW_PREF = sizeof(C) == 8 ? CM_COL_LW_F32 : CM_COL_LW_F64;
   static constexpr bool fits(int lw, int nbuf) { return smem_for(lw, nbuf) <= CM_SMEM_DYN_MAX; }
-  static constexpr bool takes(int lw) { return fits(lw, 1) && (P::TPS << lw) <= 512; }
+  static constexpr bool takes(int lw) { return fits(lw, FEW ? 2 : 1) && (P::TPS << lw) <= 512; }
   static constexpr int LW = takes(LW_PREF) ? LW_PREF : takes(LW_PREF - 1) ? LW_PREF - 1 : 0;
   static constexpr int W = 1 << LW;
   static constexpr int GROUP = W * TPS;
@@ -209,7 +215,7 @@ struct ColShape {
   // the twiddles beside one buffer they are read from the global table (ONEBUF:
   // FP64 at 2^13).
   static constexpr size_t TWS = NX * sizeof(C);
-  static constexpr bool PAIRED = CM_COL_PAIR(R, LOGX);
+  static constexpr bool PAIRED = CM_COL_PAIR(R, LOGX) && !FEW;
   static constexpr bool FIT2 = TWS + 2 * BUF <= CM_SMEM_DYN_MAX, FIT1 = TWS + BUF <= CM_SMEM_DYN_MAX;
   static constexpr bool PAIR2 = 2 * (TWS + 2 * BUF) <= CM_SMEM_DYN_MAX, PAIR1 = 2 * (TWS + BUF) <= CM_SMEM_DYN_MAX;
   static constexpr bool TWO = FIT2 && (PAIR2 || !PAIR1 || !PAIRED);
@@ -341,11 +347,11 @@ CM_DEVINL void col_pack_store(const C (&v)[E], C* __restrict__ spec, int ny, int
   }
 }
 
-template <typename R, int LOGX, int BASE = CM_COL_BASE>
-__global__ void __launch_bounds__(ColShape<R, LOGX, BASE>::THREADS, ColShape<R, LOGX, BASE>::MINB)
+template <typename R, int LOGX, int BASE = CM_COL_BASE, bool FEW = false>
+__global__ void __launch_bounds__(ColShape<R, LOGX, BASE, FEW>::THREADS, ColShape<R, LOGX, BASE, FEW>::MINB)
 k_op_col(OpArgs<R> a) {
   typedef typename CT<R>::C C;
-  typedef ColShape<R, LOGX, BASE> Sh;
+  typedef ColShape<R, LOGX, BASE, FEW> Sh;
   typedef typename Sh::P P;
   constexpr int NX = P::N, W = Sh::W, LW = Sh::LW, E = Sh::E;
   extern __shared__ __align__(16) unsigned char smem_raw[];
