@@ -63,23 +63,37 @@ int sm_count() {
 
 std::mutex g_op_mu;
 
+// whether blocks of shape Sh give every second SM a tile of so many rows
+template <typename Sh>
+bool row_blocks_many(int rows) {
+  return 2 * ((rows + 2 * Sh::NP - 1) / (2 * Sh::NP)) > sm_count();
+}
+
+template <typename R, int LOGN, bool SMALL>
+int row_fwd_as(const OpArgs<R>& a, cudaStream_t s, bool launch) {
+  typedef OpRowShape<R, LOGN, SMALL> Sh;
+  static KernelInfo info;
+  int rc;
+  {
+    std::lock_guard<std::mutex> g(g_op_mu);
+    rc = prepare<R, LOGN, decltype(&k_op_row_fwd<R, LOGN, SMALL>), Sh>(k_op_row_fwd<R, LOGN, SMALL>, info);
+  }
+  if (rc || !launch) return rc;
+  const int tiles = (a.in_rows + 2 * Sh::NP - 1) / (2 * Sh::NP);
+  const int grid = std::max(1, std::min(tiles, info.grid_per_sm * sm_count()));
+  k_op_row_fwd<R, LOGN, SMALL><<<grid, Sh::THREADS, Sh::smem(), s>>>(a);
+  return 0;
+}
+
 template <typename R, int LOGN>
 int row_fwd(const OpArgs<R>& a, cudaStream_t s, bool launch = true) {
   if constexpr (!len_fits<R, LOGN>()) {
     return -1;
   } else {
-    typedef OpRowShape<R, LOGN> Sh;
-    static KernelInfo info;
-    int rc;
-    {
-      std::lock_guard<std::mutex> g(g_op_mu);
-      rc = prepare<R, LOGN, decltype(&k_op_row_fwd<R, LOGN>), Sh>(k_op_row_fwd<R, LOGN>, info);
+    if constexpr (op_row_both<R, LOGN>()) {
+      if (row_blocks_many<OpRowShape<R, LOGN, false>>(a.in_rows)) return row_fwd_as<R, LOGN, false>(a, s, launch);
     }
-    if (rc || !launch) return rc;
-    const int tiles = (a.in_rows + 2 * Sh::NP - 1) / (2 * Sh::NP);
-    const int grid = std::max(1, std::min(tiles, info.grid_per_sm * sm_count()));
-    k_op_row_fwd<R, LOGN><<<grid, Sh::THREADS, Sh::smem(), s>>>(a);
-    return 0;
+    return row_fwd_as<R, LOGN, true>(a, s, launch);
   }
 }
 
@@ -148,23 +162,31 @@ int col(const OpArgs<R>& a, cudaStream_t s, bool launch = true) {
   }
 }
 
+template <typename R, int LOGN, bool SMALL>
+int row_inv_as(const OpArgs<R>& a, cudaStream_t s, bool launch) {
+  typedef OpRowShape<R, LOGN, SMALL> Sh;
+  static KernelInfo info;
+  int rc;
+  {
+    std::lock_guard<std::mutex> g(g_op_mu);
+    rc = prepare<R, LOGN, decltype(&k_op_row_inv<R, LOGN, SMALL>), Sh>(k_op_row_inv<R, LOGN, SMALL>, info);
+  }
+  if (rc || !launch) return rc;
+  const int tiles = (a.out_rows + 2 * Sh::NP - 1) / (2 * Sh::NP);
+  const int grid = std::max(1, std::min(tiles, info.grid_per_sm * sm_count()));
+  launch_pdl(k_op_row_inv<R, LOGN, SMALL>, grid, Sh::THREADS, Sh::smem(), s, a);
+  return 0;
+}
+
 template <typename R, int LOGN>
 int row_inv(const OpArgs<R>& a, cudaStream_t s, bool launch = true) {
   if constexpr (!len_fits<R, LOGN>()) {
     return -1;
   } else {
-    typedef OpRowShape<R, LOGN> Sh;
-    static KernelInfo info;
-    int rc;
-    {
-      std::lock_guard<std::mutex> g(g_op_mu);
-      rc = prepare<R, LOGN, decltype(&k_op_row_inv<R, LOGN>), Sh>(k_op_row_inv<R, LOGN>, info);
+    if constexpr (op_row_both<R, LOGN>()) {
+      if (row_blocks_many<OpRowShape<R, LOGN, false>>(a.out_rows)) return row_inv_as<R, LOGN, false>(a, s, launch);
     }
-    if (rc || !launch) return rc;
-    const int tiles = (a.out_rows + 2 * Sh::NP - 1) / (2 * Sh::NP);
-    const int grid = std::max(1, std::min(tiles, info.grid_per_sm * sm_count()));
-    launch_pdl(k_op_row_inv<R, LOGN>, grid, Sh::THREADS, Sh::smem(), s, a);
-    return 0;
+    return row_inv_as<R, LOGN, true>(a, s, launch);
   }
 }
 

@@ -227,17 +227,25 @@ struct ColShape {
   static size_t smem() { return SMEM; }
 };
 
-// the operator's own row passes: small blocks on short rows, for the same
-// reason as CM_COL_BASE_SHORT (a solve's row passes keep theirs, the order of
-// their sums with it)
+// The operator's own row passes: blocks of 64 threads on rows of up to 512
+// points, for the same reason as CM_COL_BASE_SHORT (a solve's row passes keep
+// theirs, the order of their sums with it).  FP64 rows of 64, 384 and 512
+// points go back to the large blocks where those give every second SM one: the
+// small ones, each with the twiddles of a row or two, are then too many (2048 x
+// 384 29.8 us, 25.1 in large blocks; 8192 x 512 146 and 131; 6144 x 64 37.6 and
+// 34.3; but 1024 x 384 22.1 and 23.1, 6144 x 256 41.7 and 43.6).
+template <typename R, int LOGN, bool SMALL = true>
+using OpRowShape = OpShape<R, LOGN, row_lr<R>(LOGN), SMALL ? 64 : 0>;
 template <typename R, int LOGN>
-using OpRowShape = OpShape<R, LOGN, row_lr<R>(LOGN), 64>;
+constexpr bool op_row_both() {
+  return sizeof(R) == 8 && (LenCode<LOGN>::N <= 64 || (LenCode<LOGN>::N > 256 && LenCode<LOGN>::N <= 512));
+}
 
-template <typename R, int LOGN>
-__global__ void __launch_bounds__(OpRowShape<R, LOGN>::THREADS, OpRowShape<R, LOGN>::MINB)
+template <typename R, int LOGN, bool SMALL = true>
+__global__ void __launch_bounds__(OpRowShape<R, LOGN, SMALL>::THREADS, OpRowShape<R, LOGN, SMALL>::MINB)
 k_op_row_fwd(OpArgs<R> a) {
   typedef typename CT<R>::C C;
-  typedef OpRowShape<R, LOGN> Sh;
+  typedef OpRowShape<R, LOGN, SMALL> Sh;
   typedef typename Sh::P P;
   constexpr int N = P::N, NP = Sh::NP;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -404,11 +412,11 @@ k_op_col(OpArgs<R> a) {
   if (a.st) pdl_trigger();
 }
 
-template <typename R, int LOGN>
-__global__ void __launch_bounds__(OpRowShape<R, LOGN>::THREADS, OpRowShape<R, LOGN>::MINB)
+template <typename R, int LOGN, bool SMALL = true>
+__global__ void __launch_bounds__(OpRowShape<R, LOGN, SMALL>::THREADS, OpRowShape<R, LOGN, SMALL>::MINB)
 k_op_row_inv(OpArgs<R> a) {
   typedef typename CT<R>::C C;
-  typedef OpRowShape<R, LOGN> Sh;
+  typedef OpRowShape<R, LOGN, SMALL> Sh;
   typedef typename Sh::P P;
   constexpr int N = P::N, NP = Sh::NP;
   extern __shared__ __align__(16) unsigned char smem_raw[];

@@ -1,6 +1,6 @@
-"""The operator's column pass on both sides of its rules for the number of
-columns (cm_op_p2.cu: few columns a block each, or groups and pairs of blocks;
-small blocks or large ones), against an FFT in numpy."""
+"""The operator's row and column passes on both sides of the rules for their
+shapes (cm_op_p2.cu: small blocks or large ones, few columns a block each, or
+groups and pairs of blocks), against an FFT in numpy."""
 import numpy as np
 import pytest
 
@@ -8,9 +8,11 @@ from oracle import contact_oracle as oc
 
 pytestmark = pytest.mark.gpu
 
-# columns of 2048, 3072, 4096 in 33 to 149 and in more groups; 512 and 768
+# rows of 64, 384 and 512 in small and in large blocks; columns of 2048, 3072
+# and 4096 in few groups and in many; columns of 512 and 768
 SIDES = [(2048, 64), (2048, 512), (2048, 768), (3072, 64), (3072, 256), (3072, 384),
-         (4096, 64), (4096, 256), (4096, 384), (512, 512), (512, 1536), (768, 96)]
+         (4096, 64), (4096, 256), (4096, 384), (512, 512), (512, 1536), (768, 96), (3072, 512),
+         (1024, 384), (1536, 384), (6144, 64), (1536, 512), (8192, 64)]
 
 
 @pytest.mark.parametrize("nb", SIDES)
