@@ -31,8 +31,8 @@ struct NvtxRange {
 
 #define CM_SMEM_ROW (64 * 1024)   // ping-pong buffers of a row tile
 #define CM_COMP_ELEMS 2048
-// domain points up to which a single solve without a hardness runs in the
-// persistent kernel (cm_solo.cuh has both sides' times)
+// domain points up to which a single solve without a hardness may run in the
+// persistent kernel (solo_pays)
 #ifndef CM_SOLO_MAX_POINTS
 #define CM_SOLO_MAX_POINTS (1u << 20)
 #endif
@@ -1205,6 +1205,39 @@ static int ccg_init(cm_plan* p, Work<R>& w, const cm_ccg_params* prm, const Solv
   return CM_OK;
 }
 
+// Whether solves of the plan without a hardness run in the persistent kernel
+// (cm_solo.cuh) rather than in launched passes; by_value: those are the
+// register-resident ones (cm_ccg_p2.cuh).  Solves of 40 iterations, launched /
+// persistent, FP64 (mixed alike), ms:
+// * both sides with register-resident transforms in the persistent kernel: 512^2
+//   of a free 256^2 to 1024 x 768 3.27 / 2.97, a free 512^2 2.76 / 2.66, but a
+//   periodic 1024^2 3.36 / 3.69;
+// * longer rows, which it transforms in shared memory: 64 x 1536 2.67 / 2.46,
+//   256 x 1536 2.89 / 2.81, but 384 x 1536 3.17 / 4.52, 64 x 2048 2.44 / 2.76, 64
+//   x 4096 3.03 / 4.83;
+// * longer columns: 2048 x 64 2.65 / 2.33, 2048 x 256 3.15 / 2.89, 3072 x 256
+//   3.79 / 3.72, but 2048 x 384 3.91 / 4.56, 4096 x 64 3.40 / 3.86;
+// * launched passes of any length (30 iterations): 1000^2 6.16 / 4.58, 2500 x 400
+//   7.22 / 6.80, 250 x 4000 6.11 / 6.05, 4000 x 100 5.23 / 4.90, but 3000 x 300
+//   7.21 / 7.78, 4000 x 150 6.06 / 7.56 (columns one at a time).
+static bool solo_pays(const cm_plan* p, bool by_value) {
+  const long points = (long)p->nx * p->ny;
+  if (points > (long)CM_SOLO_MAX_POINTS) return false;
+  if (!by_value) return p->nx <= 2560 || points <= 7L << 16;
+  auto held = [](int n) {
+    switch (len_code(n)) {
+#define CM_CASE(L) case L:
+      CM_SOLO_LEN_CASES(CM_CASE)
+#undef CM_CASE
+      return true;
+      default: return false;
+    }
+  };
+  if (!held(p->ny)) return p->ny <= 1536 && points <= 3L << 17;
+  if (!held(p->nx)) return p->nx <= 3072 && p->ny <= 256;
+  return 4L * p->tx * p->ty <= 3L << 20;
+}
+
 template <typename R>
 static int run_ccg(cm_plan* p, Work<R>& w, const cm_ccg_params* prm, const SolveInput& in,
                    double rel_pentol, double rel_forcetol, int maxiter, CcgState* fin,
@@ -1219,8 +1252,7 @@ static int run_ccg(cm_plan* p, Work<R>& w, const cm_ccg_params* prm, const Solve
   // a solve with a hardness keeps to the launched passes: its plastic mask is
   // the sign of gaps that converge to zero, so it would change with the order
   // of a sum
-  bool solo = prof_iters == 0 && !prm->has_hardness && w.tiles.generic_ok &&
-              (size_t)p->nx * p->ny <= CM_SOLO_MAX_POINTS;
+  bool solo = prof_iters == 0 && !prm->has_hardness && w.tiles.generic_ok && solo_pays(p, w.by_value);
   if (solo && !w.solo_partials) {
     // the plan's first solve of this kind (batches never need these)
     // (its launch shape for the whole domain's rows, whatever this phase updates)

@@ -37,11 +37,11 @@
 // iteration of periodic 256^2 FP64, four 30), one loop body for both operators
 // (with every pass written out and unrolled the iteration's code left the
 // instruction cache: 48 us), poll and abort in one load, and the divisions of
-// the convergence step side by side.  Per iteration, launched passes / here,
-// FP64: periodic 64^2 68 / 30 us, 256^2 76 / 31, 512^2 89 / 34, 768^2 96 / 61,
-// 1024^2 95 / 79, free 128^2 77 / 33, 512^2 81 / 61; mixed alike.  Beyond 2^20
-// domain points every SM has many tiles and the launched passes' larger
-// butterflies win.
+// the convergence step side by side.  Per iteration, FP64: periodic 64^2 30 us,
+// 256^2 31, 512^2 34, 768^2 61, free 128^2 33, 512^2 61 (launched passes 65-80);
+// mixed alike.  Where every SM has many tiles, or a long side takes the
+// transforms in shared memory, the launched passes' larger butterflies win:
+// solo_pays (cm_plan.cu) has the rule and both sides' times.
 //
 // Waits are bounded (CM_BARRIER_TIMEOUT_CYCLES): a block that gives up raises
 // the abort word, every other wait sees it, and the solve ends with
