@@ -1302,8 +1302,10 @@ static int run_ccg(cm_plan* p, Work<R>& w, const cm_ccg_params* prm, const Solve
   int every = prm->check_every;
   if (every <= 0) {
     const long work = (long)p->nx * p->ny;
-    every = solo ? CM_SOLO_ITERS
-                 : work >= (1L << 20) ? (w.by_value ? 8 : 4) : (work >= (1L << 16) ? 8 : 16);
+    every = work >= (1L << 20) ? (w.by_value ? 8 : 4) : (work >= (1L << 16) ? 8 : 16);
+    // (the clock is read between launches, so a solve with a time limit keeps
+    // to the short ones)
+    if (solo && !(prm->timeout_s > 0)) every = CM_SOLO_ITERS;
   }
   const bool observe = prm->on_iteration != nullptr && prm->iteration_forces != nullptr;
   if (observe) every = 1;

@@ -60,3 +60,22 @@ def test_route(kind, nb, persistent):
         o = oc.constrained_conjugate_gradients(ref, h, **kw)
         for k in ("x", "jac"):
             assert np.linalg.norm(r[k] - o[k]) <= 1e-10 * np.linalg.norm(o[k])
+
+
+def test_time_limit_is_read_every_few_iterations():
+    """A solve with a time limit launches the persistent kernel for a few
+    iterations at a time, and ends in the same state."""
+    import contactmechanics_b200 as cm
+    from contactmechanics_b200 import _lib
+    nb = (256, 256)
+    h = oc.self_affine(nb, (1.0, 1.0), 0.8, 0.1, seed=24)
+    sub = cm.PeriodicFFTElasticHalfSpace(nb, 1.0, (1.0, 1.0))
+    kw = dict(external_force=1e-3, pentol=1e-30, forcetol=0.0, maxiter=NIT)
+    free = cm.constrained_conjugate_gradients(sub, h, **kw)
+    n0 = _lib.lib().cm_launch_count()
+    r = cm.constrained_conjugate_gradients(sub, h, timeout=1e3, **kw)
+    launches = _lib.lib().cm_launch_count() - n0
+    n0 = _lib.lib().cm_launch_count()
+    cm.constrained_conjugate_gradients(sub, h, **kw)
+    assert launches == _lib.lib().cm_launch_count() - n0 - 1 + NIT // 8
+    assert np.array_equal(r.x, free.x) and np.array_equal(r.jac, free.jac)
