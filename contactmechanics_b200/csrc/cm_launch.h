@@ -189,10 +189,10 @@ int ccg_solo_launch(const CcgArgs<R>& a, int lx, int ly, const GenFft& gx, const
 // barriers ends after `limit` cycles; *gave_up (pinned host memory) is then set
 // and the rows that were not computed hold NaN.
 template <typename R>
-SoloPlan op_one_plan(int nx, int ny, int lx, int ly, const GenFft& gx);
+SoloPlan op_one_plan(int nx, int ny, int lx, int ly);
 template <typename R>
-int op_one_launch(const OpArgs<R>& a, int lx, int ly, const GenFft& gx, const SoloPlan& sp,
-                  GridBarrier* bar, long long limit, int* gave_up, cudaStream_t s);
+int op_one_launch(const OpArgs<R>& a, int lx, int ly, const SoloPlan& sp, GridBarrier* bar,
+                  long long limit, int* gave_up, cudaStream_t s);
 
 // The persistent batch kernel (cm_batch.cu): one launch over n jobs taken in
 // queue order `order` (next: a zeroed device counter), smem bytes of dynamic

@@ -1,5 +1,6 @@
-// The operator of a small domain with sides 2^k in one cooperative launch: the
-// row, column and inverse row passes (cm_op_p2.cuh) separated by grid barriers.
+// The operator of a small domain with sides 2^k of 64 to 1024 in one cooperative
+// launch: the row, column and inverse row passes (cm_op_p2.cuh) separated by grid
+// barriers.
 //
 // Three launches cost the host about 8 us of a call, more than the GPU needs on
 // small grids; one launch stages both twiddle tables once and crosses two
@@ -14,7 +15,29 @@
 // 22.6 / 22.9).
 #include "cm_solo.cuh"
 
+// the sides it serves
+#define CM_ONE_CASES(X) X(6) X(7) X(8) X(9) X(10)
+
 namespace {
+
+template <typename R>
+CM_DEVINL void one_stage_x(int lx, typename CT<R>::C* twx, const typename CT<R>::C* tw) {
+  switch (lx) {
+#define CM_CASE(L) case L: solo_stage_x<R, L>(twx, tw); break;
+    CM_ONE_CASES(CM_CASE)
+#undef CM_CASE
+  }
+}
+
+template <typename R>
+CM_DEVINL void one_col(int lx, const OpArgs<R>& a, const typename CT<R>::C* twx, typename CT<R>::C* bufA,
+                       typename CT<R>::C* bufB) {
+  switch (lx) {
+#define CM_CASE(L) case L: solo_col<R, L>(a, a.out_rows, twx, bufA, bufB); break;
+    CM_ONE_CASES(CM_CASE)
+#undef CM_CASE
+  }
+}
 
 // The last use of the barrier in a launch: the last block leaves it zeroed for
 // the next one (launches on the same plan follow each other, replays of a
@@ -46,21 +69,20 @@ __device__ __noinline__ void one_failed(const OpArgs<R>& a, int rows, int* gave_
 
 template <typename R, int L>
 __global__ void __launch_bounds__(T, 1)
-k_op_one(const __grid_constant__ OpArgs<R> a, const __grid_constant__ SoloX X, int elems, GridBarrier* bar,
-         long long limit, int* gave_up) {
+k_op_one(const __grid_constant__ OpArgs<R> a, int lx, int elems, GridBarrier* bar, long long limit,
+         int* gave_up) {
   typedef typename CT<R>::C C;
   typedef SoloRow<L> Sh;
   typedef typename Sh::P P;
   constexpr int N = Sh::N, NP = Sh::NP, E = Sh::E, LR = Sh::LR;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ GenFft fx;
   __shared__ int ok;
   C* twy = reinterpret_cast<C*>(smem_raw);
   C* twx = twy + N;
   C* bufA = twx + a.nx;
   C* bufB = bufA + smem_padded(elems);
   stage_twiddles<L, LR, T, false>(twy, a.twy);
-  solo_stage_x_any<R>(X, fx, twx, a.twx);
+  one_stage_x<R>(lx, twx, a.twx);
   __syncthreads();
   SoloBarrier b;
   const int s = threadIdx.x >> P::LTPS, tt = threadIdx.x & (P::TPS - 1);
@@ -87,7 +109,7 @@ k_op_one(const __grid_constant__ OpArgs<R> a, const __grid_constant__ SoloX X, i
   }
   bool alive = solo_barrier(bar, b, &ok, limit);
   if (alive) {
-    solo_col_any<R>(X, fx, a, a.out_rows, twx, bufA, bufB);
+    one_col<R>(lx, a, twx, bufA, bufB);
     alive = solo_barrier(bar, b, &ok, limit);
   }
   if (alive) {
@@ -117,17 +139,16 @@ k_op_one(const __grid_constant__ OpArgs<R> a, const __grid_constant__ SoloX X, i
 
 }  // namespace
 
-// the sides it serves
-#define CM_ONE_CASES(X) X(6) X(7) X(8) X(9) X(10)
-
 // Launch shape of the operator's kernel on a domain of length codes lx, ly;
 // grid 0 when the domain or the device does not take it.
 template <typename R>
-SoloPlan op_one_plan(int nx, int ny, int lx, int ly, const GenFft& gx) {
+SoloPlan op_one_plan(int nx, int ny, int lx, int ly) {
   SoloPlan sp;
-  const SoloX X = solo_x<R>(lx, gx);
   const int nsm = solo_sms();
-  if (!nsm || X.lx < 0 || X.lx >= 32) return sp;
+  if (!nsm || lx < 6 || lx > 10) return sp;
+  SoloX X;
+  X.lx = lx;
+  X.lw = 0;
   int per_sm = 0;
   const void* kern = nullptr;
   switch (ly) {
@@ -155,11 +176,10 @@ SoloPlan op_one_plan(int nx, int ny, int lx, int ly, const GenFft& gx) {
 }
 
 template <typename R>
-int op_one_launch(const OpArgs<R>& a, int lx, int ly, const GenFft& gx, const SoloPlan& sp,
-                  GridBarrier* bar, long long limit, int* gave_up, cudaStream_t s) {
-  const SoloX X = solo_x<R>(lx, gx);
+int op_one_launch(const OpArgs<R>& a, int lx, int ly, const SoloPlan& sp, GridBarrier* bar,
+                  long long limit, int* gave_up, cudaStream_t s) {
   switch (ly) {
-#define CM_CASE(L) case L: return solo_cooperative(k_op_one<R, L>, sp, s, a, X, sp.elems, bar, limit, gave_up);
+#define CM_CASE(L) case L: return solo_cooperative(k_op_one<R, L>, sp, s, a, lx, sp.elems, bar, limit, gave_up);
     CM_ONE_CASES(CM_CASE)
 #undef CM_CASE
     default: return -1;
@@ -167,8 +187,8 @@ int op_one_launch(const OpArgs<R>& a, int lx, int ly, const GenFft& gx, const So
 }
 
 #define CM_INST(R)                                                                    \
-  template SoloPlan op_one_plan<R>(int, int, int, int, const GenFft&);                \
-  template int op_one_launch<R>(const OpArgs<R>&, int, int, const GenFft&, const SoloPlan&, \
-                                GridBarrier*, long long, int*, cudaStream_t);
+  template SoloPlan op_one_plan<R>(int, int, int, int);                               \
+  template int op_one_launch<R>(const OpArgs<R>&, int, int, const SoloPlan&, GridBarrier*, long long, \
+                                int*, cudaStream_t);
 CM_INST(float)
 CM_INST(double)

@@ -743,7 +743,7 @@ static int init_work(cm_plan* p, Work<R>& w) {
   CK(cudaMemsetAsync(w.counter, 0, sizeof(unsigned int), p->stream));
   CKS(dalloc(p, &w.st, 1));
   if ((long)p->nx * p->ny <= CM_ONE_MAX_POINTS && w.tiles.generic_ok) {
-    w.one = op_one_plan<R>(p->nx, p->ny, len_code(p->nx), len_code(p->ny), p->gx);
+    w.one = op_one_plan<R>(p->nx, p->ny, len_code(p->nx), len_code(p->ny));
     if (w.one.grid) {
       CKS(dalloc(p, &w.one_bar, 1));
       CK(cudaMemsetAsync(w.one_bar, 0, sizeof(GridBarrier), p->stream));
@@ -896,7 +896,7 @@ static int launch_plain(cm_plan* p, Work<R>& w, int mode, int table_sel, const R
       a.cg_only = 0;
       a.fwd_real = nullptr;
       if (w.one.grid && !per_pass) {
-        if (op_one_launch<R>(a, lx, ly, p->gx, w.one, w.one_bar, w.one_limit, p->gave_up, s) == 0) {
+        if (op_one_launch<R>(a, lx, ly, w.one, w.one_bar, w.one_limit, p->gave_up, s) == 0) {
           w.one_limit = CM_BARRIER_TIMEOUT_CYCLES;
           g_launches += 1;
           return CM_OK;
