@@ -13,7 +13,7 @@
 #pragma once
 #include "cm_common.cuh"
 
-#define CM_MAX_STAGES 9  // lengths that fit shared memory (below 16384) have at most 8
+#define CM_MAX_STAGES 9  // lengths whose passes fit shared memory (up to 9386) have at most 8
 
 struct FftDesc {
   int n;

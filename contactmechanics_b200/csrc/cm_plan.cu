@@ -93,37 +93,34 @@ static cudaError_t& last_cuda_error() {
 // ---------------------------------------------------------------------------
 // FFT descriptors and twiddles
 // ---------------------------------------------------------------------------
-static bool make_fft_desc(int n, FftDesc* d) {
+// (nst = -1: more stages than a descriptor holds; no pass holds such a length,
+// and its plans keep their tables only)
+static void make_fft_desc(int n, FftDesc* d) {
   memset(d, 0, sizeof(*d));
   d->n = n;
   int m = n, k = 0;
-  // (longer lengths, whose transforms no pass holds, may run out of stages;
-  // they keep their tables only)
   auto push = [&](int r) {
-    if (k < CM_MAX_STAGES) d->rad[k++] = r;
-    return true;
+    if (k < CM_MAX_STAGES) d->rad[k] = r;
+    ++k;
+    m /= r;
   };
-  while (m % 8 == 0 && m >= 8) { if (!push(8)) return false; m /= 8; }
-  while (m % 4 == 0) { if (!push(4)) return false; m /= 4; }
-  while (m % 2 == 0) { if (!push(2)) return false; m /= 2; }
-  const int small[3] = {3, 5, 7};
-  for (int p : small)
-    while (m % p == 0) { if (!push(p)) return false; m /= p; }
-  for (int p = 11; m > 1; p += 2) {
+  while (m % 8 == 0) push(8);
+  while (m % 4 == 0) push(4);
+  while (m % 2 == 0) push(2);
+  for (int p : {3, 5, 7})
+    while (m % p == 0) push(p);
+  for (int p = 11; m > 1; p += 2)
     while (m % p == 0) {
-      if (!push(p)) return false;
+      push(p);
       d->generic = 1;
-      m /= p;
     }
-  }
-  d->nst = k;
+  d->nst = k <= CM_MAX_STAGES ? k : -1;
   int Ns = 1;
-  for (int i = 0; i < k; ++i) {
+  for (int i = 0; i < d->nst; ++i) {
     d->dm[i] = make_fastdiv((unsigned)(n / d->rad[i]));
     d->dns[i] = make_fastdiv((unsigned)Ns);
     Ns *= d->rad[i];
   }
-  return true;
 }
 
 template <typename C>
@@ -722,6 +719,7 @@ template <typename R>
 static int init_work(cm_plan* p, Work<R>& w) {
   typedef typename CT<R>::C C;
   CKS(choose_tiles(p->nx, p->ny, p->nyh, p->tx, p->ty, sizeof(C), &w.tiles));
+  w.tiles.generic_ok = w.tiles.generic_ok && p->fx.nst >= 0 && p->fy.nst >= 0;
   std::vector<C> twx = make_twiddles<C>(p->nx), twy = make_twiddles<C>(p->ny);
   CKS(dalloc(p, &w.twx, p->nx));
   CKS(dalloc(p, &w.twy, p->ny));
@@ -2033,7 +2031,8 @@ int cm_plan_create(const cm_plan_desc* desc, void* stream, cm_plan** out) {
     cm_plan_destroy(p);
     return code;
   };
-  if (!make_fft_desc(p->nx, &p->fx) || !make_fft_desc(p->ny, &p->fy)) return fail(CM_ERR_SIZE);
+  make_fft_desc(p->nx, &p->fx);
+  make_fft_desc(p->ny, &p->fy);
   make_gen_fft(p->nx, &p->gx);
   make_gen_fft(p->ny, &p->gy);
   if (stream) {
@@ -2604,7 +2603,8 @@ int cm_apply_periodic_noalloc(int nx, int ny, double sx, double sy, double young
   if (nx < 2 || ny < 2 || !(sx > 0) || !(sy > 0) || !(young > 0)) return CM_ERR_ARG;
   if (nx > CM_NOALLOC_MAX_SIDE || ny > CM_NOALLOC_MAX_SIDE) return CM_ERR_SIZE;
   FftDesc fx, fy;
-  if (!make_fft_desc(nx, &fx) || !make_fft_desc(ny, &fy)) return CM_ERR_SIZE;
+  make_fft_desc(nx, &fx);
+  make_fft_desc(ny, &fy);
   const int nyh = ny / 2 + 1;
   Tiles T;
   CKS(choose_tiles(nx, ny, nyh, nx, ny, sizeof(double2), &T));
