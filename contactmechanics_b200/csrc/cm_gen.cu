@@ -206,7 +206,7 @@ bool gen_ready() {
 // Row pairs of a tile for a pass of npairs pairs of length n: about a thousand
 // elements, so that small grids spread over the SMs (a pass of 500 x 300 has
 // 84 tiles of 3 pairs), one pair for long rows.
-int gen_row_pairs(int n, int npairs) { return std::max(1, std::min(1024 / n, npairs)); }
+static int gen_row_pairs(int n, int npairs) { return std::max(1, std::min(1024 / n, npairs)); }
 
 // log2 of the columns of a tile: 32 bytes of consecutive spectrum, fewer when
 // two buffers and the twiddles do not fit.

@@ -50,12 +50,10 @@ CM_DEVINL size_t spec_at(int x, int k, int nx, int lw) {
 // round trip), thread 0 works on that copy, and the threads write it back.  Read
 // and written field by field in global memory, the convergence step alone
 // was a dozen dependent L2 accesses.
-// tile_finish_warp hands the copy to the whole of warp 0; tile_finish to its
-// first lane.
 template <int NV, typename Fin>
-CM_DEVINL void tile_finish_warp(CcgState* __restrict__ st, double* __restrict__ partials,
-                                unsigned int* counter, int tile, int ntiles, double (&v)[NV],
-                                const int (&kinds)[NV], Fin fin) {
+CM_DEVINL void tile_finish(CcgState* __restrict__ st, double* __restrict__ partials,
+                           unsigned int* counter, int tile, int ntiles, double (&v)[NV],
+                           const int (&kinds)[NV], Fin fin) {
   __shared__ double red_sm[32 * NV];
   __shared__ __align__(16) unsigned char st_sm[sizeof(CcgState)];
   __shared__ int am_last;
@@ -80,21 +78,13 @@ CM_DEVINL void tile_finish_warp(CcgState* __restrict__ st, double* __restrict__ 
       acc[i] = red_apply(kinds[i], acc[i], __ldcg(partials + (size_t)tt * NV + i));
   }
   block_reduce<NV>(acc, kinds, red_sm);  // its barriers also publish the state's copy
-  if (threadIdx.x < 32) fin(*reinterpret_cast<CcgState*>(st_sm), acc);
-  if (threadIdx.x == 0) *counter = 0;
+  if (threadIdx.x == 0) {
+    fin(*reinterpret_cast<CcgState*>(st_sm), acc);
+    *counter = 0;
+  }
   __syncthreads();
   for (int i = threadIdx.x; i < NW; i += blockDim.x)
     reinterpret_cast<int4*>(st)[i] = reinterpret_cast<const int4*>(st_sm)[i];
-}
-
-template <int NV, typename Fin>
-CM_DEVINL void tile_finish(CcgState* __restrict__ st, double* __restrict__ partials,
-                           unsigned int* counter, int tile, int ntiles, double (&v)[NV],
-                           const int (&kinds)[NV], Fin fin) {
-  tile_finish_warp<NV>(st, partials, counter, tile, ntiles, v, kinds,
-                       [&](CcgState& s, double (&a)[NV]) {
-                         if (threadIdx.x == 0) fin(s, a);
-                       });
 }
 
 #ifndef CM_BARRIER_SLEEP_NS

@@ -116,7 +116,6 @@ struct GenFft {
 };
 void make_gen_fft(int n, GenFft* F);
 void gen_set_tile(GenFft* F, int nseq);
-int gen_row_pairs(int n, int npairs);
 template <typename R>
 int gen_col_lw(int n);
 template <typename R>
