@@ -125,6 +125,7 @@ SIGNATURES = {
                                        ctypes.c_double, _i, _vp, _vp, _vp]),
     "cm_selftest_grid_barrier": (_i, [_i, _i, ctypes.c_double, ctypes.POINTER(_i)]),
     "cm_selftest_operator_barrier": (_i, [_vp, _i, _i, ctypes.c_double]),
+    "cm_selftest_refuse_solver": (_i, [_vp, _i, _i]),
     "cm_tuning_set_tiles": (_i, [_i, _i, _i]),
     "cm_tuning_set_batch_threads": (_i, [_i, _i]),
     "cm_tuning_get": (_i, [_i, _i, ctypes.POINTER(_i), ctypes.POINTER(_i)]),

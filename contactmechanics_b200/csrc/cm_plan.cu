@@ -556,6 +556,7 @@ struct Work {
   CcgArgs<R> ccg_args{};    // their arguments
   SoloPlan solo;            // launch shape of the persistent solver (cm_solo.cu; grid 0: not used)
   double* solo_partials = nullptr;
+  int solo_refuse = -1;     // its launches until one counts as refused (cm_selftest_refuse_solver)
   SoloPlan one;             // launch shape of the one-launch operator (cm_op_one.cu)
   GridBarrier* one_bar = nullptr;
   long long one_limit = CM_BARRIER_TIMEOUT_CYCLES;  // of its next launch's waits
@@ -1313,8 +1314,9 @@ static int run_ccg(cm_plan* p, Work<R>& w, const cm_ccg_params* prm, const Solve
   const int lx = len_code(p->nx), ly = len_code(p->ny);
   for (int done_iters = 0;; done_iters += every) {
     if (solo) {
-      if (ccg_solo_launch<R>(w.ccg_args, lx, ly, p->gx, p->gy, w.solo, every, w.bar, w.solo_partials,
-                             s) == 0) {
+      const bool refuse = w.solo_refuse >= 0 && w.solo_refuse-- == 0;
+      if (!refuse && ccg_solo_launch<R>(w.ccg_args, lx, ly, p->gx, p->gy, w.solo, every, w.bar,
+                                        w.solo_partials, s) == 0) {
         g_launches += 1;
       } else {
         // the cooperative launch was refused (for example fewer SMs available
@@ -2796,6 +2798,12 @@ int cm_selftest_operator_barrier(cm_plan* p, int precision, int missing, double 
   CK(cudaDeviceSynchronize());  // no launch is at the barrier
   CK(cudaMemcpy(&bar->count, &count, sizeof(count), cudaMemcpyHostToDevice));
   (precision == CM_FP64 ? p->w64.one_limit : p->w32.one_limit) = (long long)(limit_us * 1e-3 * khz) + 1;
+  return CM_OK;
+}
+
+int cm_selftest_refuse_solver(cm_plan* p, int precision, int launches) {
+  if (!p || (precision != CM_FP64 && precision != CM_FP32) || launches < 0) return CM_ERR_ARG;
+  (precision == CM_FP64 ? p->w64.solo_refuse : p->w32.solo_refuse) = launches;
   return CM_OK;
 }
 

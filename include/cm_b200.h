@@ -366,6 +366,14 @@ int cm_selftest_grid_barrier(int blocks, int phantom, double limit_us, int* gave
 int cm_selftest_operator_barrier(cm_plan* plan, int precision, int missing, double limit_us);
 
 /*
+ * Makes the plan's solves in `precision` take the launch of the persistent
+ * solver after the next `launches` of them as refused by the device: that
+ * solve goes on, and later ones run, in launched passes.  Instrumentation; no
+ * reference counterpart.
+ */
+int cm_selftest_refuse_solver(cm_plan* plan, int precision, int launches);
+
+/*
  * Tuning of the per-pass kernels that batched solves (cm_ccg_solve_batch),
  * the stepping interface and sizes without register-resident passes (sides
  * other than 2^k and 3 * 2^m) run.
