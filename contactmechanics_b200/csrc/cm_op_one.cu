@@ -8,7 +8,7 @@
 // solver: the passes are bound by the latency of a few warps per SM and by the
 // fetch of instructions that each run once (ncu, 64^2: 8 warps wait for an
 // instruction, 5 at a barrier, per issue).  Per call,
-// one launch against three: FP64 64^2 10.5 / 15.0 us, 256^2 13.4 / 16.5,
+// one launch against three: FP64 64^2 10.9 / 15.0 us, 256^2 13.4 / 16.5,
 // 512^2 14.4 / 18.5, FP32 512^2 12.8 / 15.4; from 1024^2 on the launched
 // passes' longer butterflies win (30.8 / 24.2), as they do for sides 3 * 2^m
 // (192^2 22.0 / 18.6) and, but for the host's part, for others (500 x 300

@@ -61,7 +61,7 @@
 // FP64: 33 blocks of 256 threads, 129 of 64; plastic 512^2 solve 9.3 -> 8.5 ms,
 // operator FP64 384^2 21.6 -> 15.0 us).  With more columns the larger blocks
 // stage fewer twiddles (512 x 2048 24.9 us, 26.9 with blocks of 64); columns of
-// 3 * 2^m points keep to the small ones (768 x 1536 FP64 41.0 -> 39.2 us).
+// 3 * 2^m points keep to the small ones (768 x 1536 FP64 41.1 and 41.0 us).
 #ifndef CM_COL_BASE_SHORT
 #define CM_COL_BASE_SHORT 64
 #endif

@@ -181,8 +181,10 @@ int cm_plan_shape(const cm_plan* plan, int* nxd, int* nyd, int* nyh);
  * Which transform engine serves the plan's operator and single solves in
  * `precision` (CM_FP64 or CM_FP32): *engine = 1 for the register-resident
  * passes (domain sides 2^k and 3 * 2^m), 0 where at least one side takes the
- * shared-memory transforms of any length.  No counterpart in the reference
- * (numpy's FFT serves every size there).
+ * shared-memory transforms of any length.  (Small elastic solves run in a
+ * persistent kernel, whose register-resident transforms end at 1024 and 768
+ * points: a longer side takes those in shared memory there, engine 1 or not.)
+ * No counterpart in the reference (numpy's FFT serves every size there).
  */
 int cm_plan_engine(const cm_plan* plan, int precision, int* engine);
 
@@ -414,10 +416,8 @@ unsigned long long cm_launch_count(void);
  * eagerly with a CUDA event between kernels on the plan's stream.  Writes
  * the average milliseconds of each of the *n_kernels kernels (launch order)
  * to ms_per_kernel (capacity >= 16) and, if names is not NULL, their names.
- * Plans that run the persistent solver kernel report it as entry 0
- * ("k_ccg_persist", event-timed milliseconds per iteration) followed by its
- * phases ("k_ccg_persist:<phase>", milliseconds per iteration from
- * in-kernel timer stamps of a second run; they sum to about entry 0).
+ * The launched passes are timed on every plan, also on small domains whose
+ * elastic solves run in one persistent kernel instead.
  * Returns CM_ERR_ARG if the solve stopped before `iters` iterations.
  * Instrumentation; no reference counterpart.
  */
