@@ -17,6 +17,11 @@
 // by addition.  (Recomputing twiddled inputs and (p q) mod r inside a double
 // loop on one thread per butterfly, the 73-point stages of a 511 x 256
 // domain took 534 us a column pass; here 12.)
+// Its rounding against numpy in 64 bits, mixed-radix passes / these (medians of
+// five rough fields): displacements 1010 x 1370 FP64 8.4e-16 / 6.5e-16, 590 x 610
+// FP32 2.7e-7 / 1.8e-7; forces, whose stiffness amplifies the shortest waves,
+// 299 x 253 FP64 7.2e-15 / 6.9e-15, 1010 x 1370 3.5e-14 / 3.7e-14, 1990 x 64 (a
+// factor 199) 7.3e-14 / 8.9e-14.
 //
 // Operator FP64, mixed-radix passes / these: 500 x 300 49.2 / 22.6 us, 1000^2
 // 63.6 / 50, 167^2 2750 / 33, 511 x 256 565 / 20.5.  Bound by the stages'
